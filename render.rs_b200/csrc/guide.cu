@@ -481,33 +481,41 @@ __device__ __forceinline__ unsigned long long to_fix(float v) {
 __device__ __forceinline__ float from_fix(unsigned long long q) { return (float)(long long)q * (1.0f / G_FIX_SCALE); }
 
 // ---- hash-grid backward ---------------------------------------------------------
-__global__ void k_guide_hash_bwd(GuideDev G, const float* __restrict__ rec, const float* __restrict__ dX0, uint32_t n,
-                                 BatchSel B, unsigned long long* gtable) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, begin;
+// One warp per record, two levels at a time: lane = (level of the pair,
+// corner, feature). The 16 sums of a level fall into 128-byte blocks of the
+// gradient table (2x2x2 vertices x 2 features x 8 B), so the atomics of a warp
+// leave as a few sectors. Bound by the L2's atomic units: with a thread per
+// record, every lane's word was a request of its own (65,536 records: 84 us,
+// now 44).
+constexpr int HB_WARPS = 8;
+__global__ void __launch_bounds__(32 * HB_WARPS) k_guide_hash_bwd(GuideDev G, const float* __restrict__ rec,
+                                                                  const float* __restrict__ dX0, uint32_t n, BatchSel B,
+                                                                  unsigned long long* gtable) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t i = blockIdx.x * HB_WARPS + (threadIdx.x >> 5);
+    uint32_t begin;
     n = batch_slice(B, n, begin);
     rec += 16 * (size_t)begin;
     if (i >= n) return;
     const float* r = rec + 16 * (size_t)i;
-    float3 pn = guide_normalize_pos(G, f3(r[0], r[1], r[2]));
-    const float* dx = dX0 + 32 * (size_t)i;
-    for (int l = 0; l < G_LEVELS; l++) {
-        float rs = G.res[l];
-        uint32_t res1 = (uint32_t)rs + 2u;
-        bool dense = grid_dense(res1);
-        float fx = pn.x * rs, fy = pn.y * rs, fz = pn.z * rs;
-        float ix = floorf(fx), iy = floorf(fy), iz = floorf(fz);
-        float tx = fx - ix, ty = fy - iy, tz = fz - iz;
-        uint32_t x0 = (uint32_t)ix, y0 = (uint32_t)iy, z0 = (uint32_t)iz;
-        float g0 = dx[2 * l], g1 = dx[2 * l + 1];
-        unsigned long long* T = gtable + (size_t)l * G_T * 2;
-        for (int c = 0; c < 8; c++) {
-            uint32_t ddx = c & 1, ddy = (c >> 1) & 1, ddz = (c >> 2) & 1;
-            float w = (ddx ? tx : 1.f - tx) * (ddy ? ty : 1.f - ty) * (ddz ? tz : 1.f - tz);
-            uint32_t idx = grid_index(x0 + ddx, y0 + ddy, z0 + ddz, res1, dense);
-            const float a = w * g0, b = w * g1;
-            if (a != 0.f) atomicAdd(T + 2 * (size_t)idx, to_fix(a));
-            if (b != 0.f) atomicAdd(T + 2 * (size_t)idx + 1, to_fix(b));
-        }
+    const float3 pn = guide_normalize_pos(G, f3(r[0], r[1], r[2]));
+    const float grad = dX0[32 * (size_t)i + lane];
+    const uint32_t feat = lane & 1u, ddx = (lane >> 1) & 1u, ddy = (lane >> 2) & 1u, ddz = (lane >> 3) & 1u,
+                   half = lane >> 4;
+#pragma unroll
+    for (int it = 0; it < G_LEVELS / 2; it++) {
+        const float rs = half ? G.res[2 * it + 1] : G.res[2 * it];
+        const uint32_t res1 = (uint32_t)rs + 2u;
+        const bool dense = grid_dense(res1);
+        const float fx = pn.x * rs, fy = pn.y * rs, fz = pn.z * rs;
+        const float ix = floorf(fx), iy = floorf(fy), iz = floorf(fz);
+        const float tx = fx - ix, ty = fy - iy, tz = fz - iz;
+        const uint32_t x0 = (uint32_t)ix, y0 = (uint32_t)iy, z0 = (uint32_t)iz;
+        const float g = __shfl_sync(0xFFFFFFFFu, grad, 4 * it + 2 * half + feat);
+        const float w = (ddx ? tx : 1.f - tx) * (ddy ? ty : 1.f - ty) * (ddz ? tz : 1.f - tz);
+        const uint32_t idx = grid_index(x0 + ddx, y0 + ddy, z0 + ddz, res1, dense);
+        const float v = w * g;
+        if (v != 0.f) atomicAdd(gtable + ((size_t)(2 * it + half) * G_T + idx) * 2 + feat, to_fix(v));
     }
 }
 
@@ -548,25 +556,39 @@ __global__ void k_guide_adam_mlp(AdamArgs A, float* p, float* g, float* m, float
     if (i < n_weights) w16[i] = __float2bfloat16_rn(pi);
 }
 
-__global__ void k_guide_adam_table(AdamArgs A, float* p, unsigned long long* g, float* m, float* v, __half* t16,
-                                   uint32_t n) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || A.c[2] == 0.f) return;
+// Lazy (sparse) Adam: a table entry no record touched this step keeps its
+// parameter and moments. A thread reads four gradients (32 bytes) and touches
+// the rest of its entries only if one of them is not zero. Bound by HBM (the
+// 134 MB of gradients are read, the touched entries' state moved): with one
+// entry per thread too few bytes were in flight (106 us a step, now 70).
+__global__ void __launch_bounds__(256) k_guide_adam_table(AdamArgs A, float4* __restrict__ p, ulonglong2* __restrict__ g,
+                                                          float4* __restrict__ m, float4* __restrict__ v,
+                                                          uint2* __restrict__ t16, uint32_t n4) {
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n4 || A.c[2] == 0.f) return;
+    const ulonglong2 g0 = g[2 * (size_t)i], g1 = g[2 * (size_t)i + 1];
+    if ((g0.x | g0.y | g1.x | g1.y) == 0ull) return;
     const float c1 = A.c[0], c2 = A.c[1];
-    // Lazy (sparse) Adam: a table entry no record touched this step keeps its
-    // parameter and moments. A batch touches a few percent of the 16M
-    // entries, so the step reads the gradient table and updates only those.
-    const unsigned long long q = g[i];
-    if (q == 0ull) return;
-    float gi = from_fix(q);
-    float mi = A.b1 * m[i] + (1.f - A.b1) * gi;
-    float vi = A.b2 * v[i] + (1.f - A.b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    float pi = p[i] - A.lr * (mi * c1) / (sqrtf(vi * c2) + A.eps);
-    p[i] = pi;
-    g[i] = 0ull;
-    t16[i] = __float2half_rn(pi);
+    const unsigned long long q[4] = {g0.x, g0.y, g1.x, g1.y};
+    const float4 p4 = p[i], m4 = m[i], v4 = v[i];
+    const uint2 t4 = t16[i];
+    float pv[4] = {p4.x, p4.y, p4.z, p4.w}, mv[4] = {m4.x, m4.y, m4.z, m4.w}, vv[4] = {v4.x, v4.y, v4.z, v4.w};
+    uint32_t h[4] = {t4.x & 0xFFFFu, t4.x >> 16, t4.y & 0xFFFFu, t4.y >> 16};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (q[k] == 0ull) continue;
+        const float gi = from_fix(q[k]);
+        mv[k] = A.b1 * mv[k] + (1.f - A.b1) * gi;
+        vv[k] = A.b2 * vv[k] + (1.f - A.b2) * gi * gi;
+        pv[k] = pv[k] - A.lr * (mv[k] * c1) / (sqrtf(vv[k] * c2) + A.eps);
+        h[k] = __half_as_ushort(__float2half_rn(pv[k]));
+    }
+    p[i] = make_float4(pv[0], pv[1], pv[2], pv[3]);
+    m[i] = make_float4(mv[0], mv[1], mv[2], mv[3]);
+    v[i] = make_float4(vv[0], vv[1], vv[2], vv[3]);
+    t16[i] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+    g[2 * (size_t)i] = make_ulonglong2(0ull, 0ull);
+    g[2 * (size_t)i + 1] = make_ulonglong2(0ull, 0ull);
 }
 
 // ---- tcgen05 GEMM self-test: D[128][N] = A[128][K] B[N][K]^T -------------------------------
@@ -709,7 +731,7 @@ static int launch_backward(rt_guide* g, const float* rec, uint32_t n, cudaStream
     k_guide_bwd<<<grid, TILE, B_BYTES, st>>>(g->G, g->X0, g->acts, g->out, rec, n, B, g->part, g->dX0, g->loss,
                                              g->err);
     k_guide_grad_reduce<<<(G_NPARAMS + 255) / 256, 256, 0, st>>>(g->part, grid, g->gw);
-    k_guide_hash_bwd<<<(n + 127) / 128, 128, 0, st>>>(g->G, rec, g->dX0, n, B, g->gt);
+    k_guide_hash_bwd<<<(n + HB_WARPS - 1) / HB_WARPS, 32 * HB_WARPS, 0, st>>>(g->G, rec, g->dX0, n, B, g->gt);
     G_TRY(cudaGetLastError());
     return 0;
 }
@@ -720,7 +742,9 @@ static void launch_adam(rt_guide* g, uint32_t n, cudaStream_t st, BatchSel B = B
     k_guide_adam_mlp<<<(G_NPARAMS + 255) / 256, 256, 0, st>>>(A, g->w32, g->gw, g->mw, g->vw, g->w16, G_NWEIGHTS,
                                                              G_NPARAMS);
     uint32_t tn = (uint32_t)(G_LEVELS * G_T * 2);
-    k_guide_adam_table<<<(tn + 255) / 256, 256, 0, st>>>(A, g->t32, g->gt, g->mt, g->vt, g->t16, tn);
+    const uint32_t n4 = tn / 4;
+    k_guide_adam_table<<<(n4 + 255) / 256, 256, 0, st>>>(A, (float4*)g->t32, (ulonglong2*)g->gt, (float4*)g->mt,
+                                                         (float4*)g->vt, (uint2*)g->t16, n4);
 }
 
 // ---- entry points for the renderer (guide_internal.h) ------------------------------
