@@ -87,14 +87,6 @@ __device__ void stage_matrix(uint8_t* dst, const __nv_bfloat16* src, int R, int 
         *reinterpret_cast<uint4*>(dst + core_offset(r, kc * 8, K)) = v;
     }
 }
-// Copy the transpose of a row-major [R][K] bf16 matrix (i.e. a [K][R] operand).
-__device__ void stage_transpose(uint8_t* dst, const __nv_bfloat16* src, int R, int K) {
-    for (int i = threadIdx.x; i < R * K; i += blockDim.x) {
-        int r = i / K, k = i % K;
-        *reinterpret_cast<__nv_bfloat16*>(dst + core_offset(k, r, R)) = src[i];
-    }
-}
-
 }  // namespace
 
 // ---- encode -------------------------------------------------------------------
@@ -283,58 +275,68 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) k_guide_fwd(GuideDev G, const 
 }
 
 // ---- backward -----------------------------------------------------------------
-// Shared memory: WT0 [48][64] 6144 | WT1 8192 | WT2 8192 | WT3 [64][48] 6144 |
-//                DZ [128][64] 16384 | DZT [128][128] 32768 | HT [80][128] 20480
-// HT holds the layer input transposed plus one row of ones and zero rows up
-// to K_in + 16: the dW GEMM then also yields column K_in = sum over the batch
-// of dZ, the bias gradient (no per-neuron warp reductions).
-// TMEM: dW (and the bias column) in columns [0, 80), dH in [128, 192).
-constexpr int B_WT0 = 0, B_WT1 = 6144, B_WT2 = B_WT1 + 8192, B_WT3 = B_WT2 + 8192, B_DZ = B_WT3 + 6144,
-              B_DZT = B_DZ + 16384, B_HT = B_DZT + 32768, B_BYTES = B_HT + 20480;
-constexpr uint32_t B_TMEM_DH = 128;
+// One persistent CTA per SM runs BWD_GROUPS tile pipelines (one warpgroup each)
+// over weights they share, as the forward does. Per layer a pipeline stores dZ
+// and the layer's input H once, row by row in the core-matrix layout, and
+// issues both GEMMs on them: dH = dZ W reads dZ K-major, dW = dZ^T H reads dZ
+// and H transposed (MN-major descriptors over the same bytes), so nothing is
+// copied transposed. With M = 128 the dW GEMM also reads the 64 columns past
+// dZ's last neuron (bytes of the next rows, at the end of the H buffer):
+// accumulator rows nobody reads. The bias gradients are column sums of dZ.
+// A pipeline adds its tiles' dW / db into its own partial row, which is laid out
+// [input][neuron] so the neurons of a warp's lanes are neighbours;
+// k_guide_grad_reduce adds the rows in a fixed order.
+// The pass is latency-bound (a chain of four GEMM pairs per tile, nothing near a
+// peak): transposed copies of dZ and H written two bytes at a time, row-strided
+// global sums and two one-tile CTAs per SM took 186 us for 65,536 records; this
+// takes 43.
+// Shared memory: W0 6144 | W1 8192 | W2 8192 | W3 6144 | per group DZ 16384, H 16384.
+// TMEM per group: dW in columns [0, 64), dH in [64, 128).
+constexpr int BWD_GROUPS = 4, BWD_THREADS = BWD_GROUPS * TILE;
+constexpr uint32_t BWD_TMEM_COLS = 128 * BWD_GROUPS;
+constexpr int B_ACT = F_ACT, B_BYTES = B_ACT + BWD_GROUPS * 32768;
+static_assert(BWD_TMEM_COLS == 512, "backward: TMEM allocation is a power of two");
 
-__global__ void __launch_bounds__(TILE) k_guide_bwd(GuideDev G, const __nv_bfloat16* __restrict__ X0,
-                                                    const __nv_bfloat16* __restrict__ acts,
-                                                    const float* __restrict__ out, const float* __restrict__ rec,
-                                                    uint32_t n, BatchSel B, float* part,
-                                                    float* dX0, float* loss_sum, uint32_t* err) {
+__global__ void __launch_bounds__(BWD_THREADS, 1) k_guide_bwd(GuideDev G, const __nv_bfloat16* __restrict__ X0,
+                                                              const __nv_bfloat16* __restrict__ acts,
+                                                              const float* __restrict__ out,
+                                                              const float* __restrict__ rec, uint32_t n, BatchSel B,
+                                                              float* part, float* dX0, float* loss_sum, uint32_t* err) {
     uint32_t begin;
     n = batch_slice(B, n, begin);
+    if ((uint64_t)blockIdx.x * TILE >= n) return;  // no tile for this CTA
     rec += 16 * (size_t)begin;
-    // This CTA's row of dW / db partial sums (weights, then biases): its
-    // tiles add into it in tile order; k_guide_grad_reduce adds the rows.
-    float* gW = part + (size_t)blockIdx.x * G_NPARAMS;
-    float* gb = gW + G_NWEIGHTS;
-    for (int i = threadIdx.x; i < G_NPARAMS; i += blockDim.x) gW[i] = 0.f;
-    __syncthreads();
-    if ((uint64_t)blockIdx.x * TILE >= n) return;
     extern __shared__ __align__(1024) uint8_t sm[];
-    __shared__ uint64_t mbar;
+    __shared__ uint64_t mbar[BWD_GROUPS];
     __shared__ uint32_t tmem_base;
-    __shared__ float red[TILE / 32];
-    const int tid = threadIdx.x, warp = tid >> 5;
-    for (int l = 0; l < 4; l++) {
-        const uint32_t dst = l == 0 ? B_WT0 : l == 1 ? B_WT1 : l == 2 ? B_WT2 : B_WT3;
-        stage_transpose(sm + dst, G.w + w_off(l), l_out(l), l_in(l));
+    __shared__ uint32_t group_failed[BWD_GROUPS];
+    __shared__ float red[BWD_THREADS / 32];
+    __shared__ float db_half[BWD_GROUPS][64];
+    const int tid = threadIdx.x, warp = tid >> 5, grp = tid / TILE, gt = tid % TILE;
+    stage_matrix(sm + F_W0, G.w + w_off(0), G_HID, G_IN);
+    stage_matrix(sm + F_W1, G.w + w_off(1), G_HID, G_HID);
+    stage_matrix(sm + F_W2, G.w + w_off(2), G_HID, G_HID);
+    stage_matrix(sm + F_W3, G.w + w_off(3), G_OUT, G_HID);
+    if (warp == 0) tmem_alloc(&tmem_base, BWD_TMEM_COLS);
+    if (tid < BWD_GROUPS) {
+        mbar_init(&mbar[tid], 1);
+        group_failed[tid] = 0;
     }
-    for (int i = tid; i < 32768 / 16; i += TILE) reinterpret_cast<uint4*>(sm + B_DZT)[i] = make_uint4(0, 0, 0, 0);
-    // HT rows 64..79 (layers with K_in = 64): a row of ones, then zeros.
-    for (int k = 64; k < 80; k++)
-        *reinterpret_cast<__nv_bfloat16*>(sm + B_HT + core_offset(k, tid, TILE)) = __float2bfloat16_rn(k == 64 ? 1.f : 0.f);
-    if (warp == 0) tmem_alloc(&tmem_base, 256);
-    if (tid == 0) mbar_init(&mbar, 1);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tb = tmem_base;
-    const uint32_t lane_addr = tb + ((uint32_t)(warp * 32) << 16);
+    const uint32_t acc = tmem_base + 128u * grp;
+    const uint32_t lane_addr = acc + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t s0 = smem_u32(sm);
+    const uint32_t dz_off = B_ACT + 32768u * grp, h_off = dz_off + 16384u;
+    float* gW = part + (size_t)(grp * gridDim.x + blockIdx.x) * G_NPARAMS;
+    float* gb = gW + G_NWEIGHTS;
     uint32_t phase = 0;
-    bool failed = false;
+    bool failed = false, first = true;
     float loss = 0.f;
-    for (uint32_t tile = blockIdx.x; tile * TILE < n && !failed; tile += gridDim.x) {
-        uint32_t row = tile * TILE + tid;
-        bool valid = row < n;
+    for (uint32_t tile = grp * gridDim.x + blockIdx.x; tile * TILE < n; tile += gridDim.x * BWD_GROUPS) {
+        const uint32_t row = tile * TILE + gt;
+        const bool valid = row < n;
         float dz[64];
         if (valid) {
             float o[G_OUT];
@@ -353,122 +355,160 @@ __global__ void __launch_bounds__(TILE) k_guide_bwd(GuideDev G, const __nv_bfloa
 #pragma unroll
             for (int k = 0; k < 64; k++) dz[k] = 0.f;
         }
-        for (int l = 3; l >= 0 && !failed; l--) {
+#pragma unroll
+        for (int l = 3; l >= 0; l--) {
             const int K_in = l_in(l), N_out = l_out(l);
-            // dZ (K-major over N_out) and dZ^T (rows = neurons, K = batch).
+            // dZ and the layer input H, rows of this tile. H keeps 64 columns a
+            // row in every layer: with another stride in layer 0 a thread's row
+            // would land on rows whose ReLU masks others still read.
 #pragma unroll
             for (int c = 0; c < 8; c++)
-                if (8 * c < N_out) {
-                    uint4 q = make_uint4(pack_bf16(dz[8 * c], dz[8 * c + 1]), pack_bf16(dz[8 * c + 2], dz[8 * c + 3]),
-                                         pack_bf16(dz[8 * c + 4], dz[8 * c + 5]), pack_bf16(dz[8 * c + 6], dz[8 * c + 7]));
-                    *reinterpret_cast<uint4*>(sm + B_DZ + core_offset(tid, 8 * c, N_out)) = q;
-                }
+                if (8 * c < N_out)
+                    *reinterpret_cast<uint4*>(sm + dz_off + core_offset(gt, 8 * c, N_out)) =
+                        make_uint4(pack_bf16(dz[8 * c], dz[8 * c + 1]), pack_bf16(dz[8 * c + 2], dz[8 * c + 3]),
+                                   pack_bf16(dz[8 * c + 4], dz[8 * c + 5]), pack_bf16(dz[8 * c + 6], dz[8 * c + 7]));
+            const uint4* hp = l > 0 ? reinterpret_cast<const uint4*>(acts + ((size_t)row * 3 + (l - 1)) * G_HID)
+                                    : reinterpret_cast<const uint4*>(X0 + (size_t)row * G_IN);
 #pragma unroll
-            for (int k = 0; k < 64; k++)
-                if (k < N_out) *reinterpret_cast<__nv_bfloat16*>(sm + B_DZT + core_offset(k, tid, TILE)) = __float2bfloat16_rn(dz[k]);
-            // Layer input H (rows of this tile) -> registers and H^T operand.
-            float h[64];
-            if (l > 0) {
-                const uint4* hp = reinterpret_cast<const uint4*>(acts + ((size_t)row * 3 + (l - 1)) * G_HID);
-#pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    uint4 q = valid ? hp[c] : make_uint4(0, 0, 0, 0);
-                    __nv_bfloat162 p2[4];
-                    memcpy(p2, &q, 16);
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        float2 f = __bfloat1622float2(p2[e]);
-                        h[8 * c + 2 * e] = f.x;
-                        h[8 * c + 2 * e + 1] = f.y;
-                    }
-                }
-            } else {
-                const uint4* hp = reinterpret_cast<const uint4*>(X0 + (size_t)row * G_IN);
-#pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    uint4 q = (valid && c < G_IN / 8) ? hp[c] : make_uint4(0, 0, 0, 0);
-                    __nv_bfloat162 p2[4];
-                    memcpy(p2, &q, 16);
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        float2 f = __bfloat1622float2(p2[e]);
-                        h[8 * c + 2 * e] = f.x;
-                        h[8 * c + 2 * e + 1] = f.y;
-                    }
-                }
-            }
-            // H^T rows 0..K_in-1, then (layer 0) a row of ones and zeros up to
-            // row 63; for K_in = 64 the ones row 64 and zeros were set up front.
-#pragma unroll
-            for (int k = 0; k < 64; k++) {
-                const float hv = k < K_in ? h[k] : (k == K_in ? 1.f : 0.f);
-                *reinterpret_cast<__nv_bfloat16*>(sm + B_HT + core_offset(k, tid, TILE)) = __float2bfloat16_rn(hv);
-            }
+            for (int c = 0; c < 8; c++)
+                if (8 * c < K_in)
+                    *reinterpret_cast<uint4*>(sm + h_off + core_offset(gt, 8 * c, G_HID)) =
+                        valid ? hp[c] : make_uint4(0, 0, 0, 0);
             fence_proxy_async_smem();
-            __syncthreads();
-            if (tid == 0) {
+            group_sync(grp);
+            if (gt == 0) {
                 tc_fence_after();
-                // dW[n][k] = sum_m dZ[m][n] H[m][k]  (M = 128 padded neurons, N = K_in + 16, K = batch);
-                // column K_in is the bias gradient.
-                tc_gemm_issue(tb, s0 + B_DZT, s0 + B_HT, K_in + 16, TILE, false);
+                const uint32_t w = s0 + (l == 0 ? F_W0 : l == 1 ? F_W1 : l == 2 ? F_W2 : F_W3);
                 // dH[m][k] = sum_n dZ[m][n] W[n][k]  (N = K_in, K = N_out)
-                const uint32_t wt = l == 0 ? B_WT0 : l == 1 ? B_WT1 : l == 2 ? B_WT2 : B_WT3;
-                tc_gemm_issue(tb + B_TMEM_DH, s0 + B_DZ, s0 + wt, K_in, N_out, false);
-                tc_commit(&mbar);
+                tc_gemm_issue_ops(acc + 64u, umma_k_major(s0 + dz_off, N_out), umma_transposed(w, K_in), K_in, N_out);
+                // dW[n][k] = sum_m dZ[m][n] H[m][k]  (M = neurons, N = K_in, K = batch)
+                tc_gemm_issue_ops(acc, umma_transposed(s0 + dz_off, N_out), umma_transposed(s0 + h_off, G_HID), K_in,
+                                  TILE);
+                tc_commit(&mbar[grp]);
             }
-            bool ok = mbar_wait_or_drain(&mbar, phase, G.wait_polls);
+            // db: thread pairs sum a neuron's column, 64 rows each, while the MMAs run.
+            float db = 0.f;
+            const int nn = gt & 63, m0 = (gt >> 6) * 64;
+            if (nn < N_out)
+#pragma unroll 8
+                for (int m = 0; m < 64; m++)
+                    db += __bfloat162float(
+                        *reinterpret_cast<const __nv_bfloat16*>(sm + dz_off + core_offset(m0 + m, nn, N_out)));
+            if (m0) db_half[grp][nn] = db;
+            if (!mbar_wait_or_drain(&mbar[grp], phase, G.wait_polls)) group_failed[grp] = 1;
             phase ^= 1u;
-            if (__syncthreads_or(!ok)) {
+            group_sync(grp);
+            if (group_failed[grp]) {
                 failed = true;
                 break;
             }
             tc_fence_after();
-            float v[64], vb[16];
+            if (gt < 64) {
+                // dW: lane = neuron; column k of the accumulator is input k
+                // (the last 16 of 64 are stale in layer 0, which has 48).
+                float* g = gW + w_off(l) + gt;
 #pragma unroll
-            for (int c = 0; c < 4; c++)
-                if (c * 16 < K_in) tmem_ld16(lane_addr + c * 16, v + 16 * c);
-            tmem_ld16(lane_addr + K_in, vb);
-            if (tid < N_out) {
-                float* g = gW + w_off(l) + (size_t)tid * K_in;
+                for (int h = 0; h < 2; h++) {
+                    uint32_t r[32];
+                    tmem_ld32(lane_addr + 32 * h, r);
+                    if (gt < N_out) {
 #pragma unroll
-                for (int k = 0; k < 64; k++)
-                    if (k < K_in) g[k] += v[k];
-                gb[b_off(l) + tid] += vb[0];
+                        for (int k = 0; k < 32; k++)
+                            if (32 * h + k < K_in) {
+                                const float v = __uint_as_float(r[k]);
+                                float* at = g + (32 * h + k) * N_out;
+                                *at = first ? v : *at + v;
+                            }
+                    }
+                    __syncwarp();
+                }
+                if (gt < N_out) {
+                    const float b = db + db_half[grp][gt];
+                    gb[b_off(l) + gt] = first ? b : gb[b_off(l) + gt] + b;
+                }
+                __syncwarp();
             }
 #pragma unroll
-            for (int c = 0; c < 4; c++)
-                if (c * 16 < K_in) tmem_ld16(lane_addr + B_TMEM_DH + c * 16, v + 16 * c);
-            if (l > 0) {
+            for (int h = 0; h < (l > 0 ? 2 : 1); h++) {
+                uint32_t r[32];
+                tmem_ld32(lane_addr + 64 + 32 * h, r);
+                if (l > 0) {
+                    // dZ of the layer below: dH where its ReLU passed (its bf16
+                    // activations are positive unless the bits are zero).
 #pragma unroll
-                for (int k = 0; k < 64; k++) dz[k] = h[k] > 0.f ? v[k] : 0.f;
-            } else if (valid) {
-                float4* d = reinterpret_cast<float4*>(dX0 + (size_t)row * 32);
+                    for (int c = 0; c < 4; c++) {
+                        const uint4 q =
+                            *reinterpret_cast<const uint4*>(sm + h_off + core_offset(gt, 32 * h + 8 * c, G_HID));
+                        const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-                for (int c = 0; c < 8; c++) d[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+                        for (int e = 0; e < 4; e++) {
+                            const int k = 8 * c + 2 * e;
+                            dz[32 * h + k] = (w4[e] & 0x7FFFu) ? __uint_as_float(r[k]) : 0.f;
+                            dz[32 * h + k + 1] = (w4[e] & 0x7FFF0000u) ? __uint_as_float(r[k + 1]) : 0.f;
+                        }
+                    }
+                } else if (valid) {
+                    float4* d = reinterpret_cast<float4*>(dX0 + (size_t)row * 32);
+#pragma unroll
+                    for (int c = 0; c < 8; c++)
+                        d[c] = make_float4(__uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]),
+                                           __uint_as_float(r[4 * c + 2]), __uint_as_float(r[4 * c + 3]));
+                }
             }
+            __syncwarp();
             tc_fence_before();
-            __syncthreads();
         }
+        if (failed) {
+            if (gt == 0) atomicOr(err, GERR_WAIT);
+            break;
+        }
+        first = false;
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, off);
     if ((tid & 31) == 0) red[warp] = loss;
     __syncthreads();
-    if (tid == 0) atomicAdd(loss_sum, red[0] + red[1] + red[2] + red[3]);
-    if (failed && tid == 0) atomicOr(err, GERR_WAIT);
+    if (tid == 0) {
+        float s = 0.f;
+        for (int w = 0; w < BWD_THREADS / 32; w++) s += red[w];
+        atomicAdd(loss_sum, s);
+    }
     if (warp == 0) {
-        tmem_dealloc(tb, 256);
+        tc_fence_after();
+        tmem_dealloc(tmem_base, BWD_TMEM_COLS);
         tmem_relinquish();
     }
 }
 
-// Adds the backward CTAs' partial rows to the MLP gradient, in CTA order.
-__global__ void k_guide_grad_reduce(const float* __restrict__ part, int rows, float* gw) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= G_NPARAMS) return;
+// Adds the pipelines' partial rows (one per tile, at most max_rows) to the MLP
+// gradient: eight threads a parameter take every eighth row, then their sums
+// are added in order. Rows of a failed backward pass are left out.
+constexpr int GR_PARAMS = 64, GR_SLICES = 8;
+__global__ void __launch_bounds__(GR_PARAMS* GR_SLICES) k_guide_grad_reduce(const float* __restrict__ part, uint32_t n,
+                                                                            BatchSel B, uint32_t max_rows, float* gw,
+                                                                            const uint32_t* __restrict__ err) {
+    __shared__ float sum[GR_SLICES][GR_PARAMS];
+    uint32_t begin;
+    n = batch_slice(B, n, begin);
+    const uint32_t rows = min((n + TILE - 1) / TILE, max_rows);
+    const uint32_t c = threadIdx.x % GR_PARAMS, sl = threadIdx.x / GR_PARAMS;
+    const uint32_t i = blockIdx.x * GR_PARAMS + c;
     float s = 0.f;
-    for (int b = 0; b < rows; b++) s += part[(size_t)b * G_NPARAMS + i];
-    gw[i] += s;
+    if (i < (uint32_t)G_NPARAMS && *err == 0u)
+#pragma unroll 8
+        for (uint32_t b = sl; b < rows; b += GR_SLICES) s += part[(size_t)b * G_NPARAMS + i];
+    sum[sl][c] = s;
+    __syncthreads();
+    if (sl != 0 || i >= (uint32_t)G_NPARAMS) return;
+    for (int k = 1; k < GR_SLICES; k++) s += sum[k][c];
+    // Weights come as [input][neuron] per layer.
+    uint32_t to = i;
+    if (i < (uint32_t)G_NWEIGHTS) {
+        const int l = i < (uint32_t)w_off(1) ? 0 : i < (uint32_t)w_off(2) ? 1 : i < (uint32_t)w_off(3) ? 2 : 3;
+        const uint32_t j = i - w_off(l), N_out = l_out(l), k = j / N_out, nn = j % N_out;
+        to = w_off(l) + nn * l_in(l) + k;
+    }
+    gw[to] += s;
 }
 
 // Table gradients are summed as integers in units of 2^-24 (each
@@ -641,8 +681,7 @@ struct rt_guide {
     __nv_bfloat16* w16 = nullptr;
     float* t32 = nullptr;      // table master (levels * T * 2)
     unsigned long long* gt = nullptr;  // table gradient, 2^-24 fixed point
-    float* part = nullptr;     // backward CTAs' dW / db partial rows (bwd_rows x G_NPARAMS)
-    int bwd_rows = 0;
+    float* part = nullptr;     // backward pipelines' dW / db partial rows (sms x BWD_GROUPS x G_NPARAMS)
     float* mt = nullptr;
     float* vt = nullptr;
     __half* t16 = nullptr;
@@ -726,11 +765,12 @@ static int launch_forward(rt_guide* g, const float* rec, uint32_t n, int mode, c
 static int launch_backward(rt_guide* g, const float* rec, uint32_t n, cudaStream_t st,
                            BatchSel B = BatchSel{nullptr, 0, 1}) {
     uint32_t tiles = (n + TILE - 1) / TILE;
-    int grid = (int)std::min<uint32_t>(tiles, (uint32_t)g->bwd_rows);
+    int grid = (int)std::min<uint32_t>(tiles, (uint32_t)g->sms);
     G_TRY(cudaMemsetAsync(g->loss, 0, 4, st));
-    k_guide_bwd<<<grid, TILE, B_BYTES, st>>>(g->G, g->X0, g->acts, g->out, rec, n, B, g->part, g->dX0, g->loss,
-                                             g->err);
-    k_guide_grad_reduce<<<(G_NPARAMS + 255) / 256, 256, 0, st>>>(g->part, grid, g->gw);
+    k_guide_bwd<<<grid, BWD_THREADS, B_BYTES, st>>>(g->G, g->X0, g->acts, g->out, rec, n, B, g->part, g->dX0, g->loss,
+                                                    g->err);
+    k_guide_grad_reduce<<<(G_NPARAMS + GR_PARAMS - 1) / GR_PARAMS, GR_PARAMS * GR_SLICES, 0, st>>>(
+        g->part, n, B, (uint32_t)grid * BWD_GROUPS, g->gw, g->err);
     k_guide_hash_bwd<<<(n + HB_WARPS - 1) / HB_WARPS, 32 * HB_WARPS, 0, st>>>(g->G, rec, g->dX0, n, B, g->gt);
     G_TRY(cudaGetLastError());
     return 0;
@@ -814,8 +854,7 @@ int rt_guide_create(const float* lo, const float* hi, uint64_t seed, float lr, r
     rc = rc ? rc : g->alloc(&g->w16, G_NWEIGHTS);
     rc = rc ? rc : g->alloc(&g->t32, tn);
     rc = rc ? rc : g->alloc(&g->gt, tn);
-    g->bwd_rows = g->sms * 2;
-    rc = rc ? rc : g->alloc(&g->part, (size_t)g->bwd_rows * G_NPARAMS);
+    rc = rc ? rc : g->alloc(&g->part, (size_t)g->sms * BWD_GROUPS * G_NPARAMS);
     rc = rc ? rc : g->alloc(&g->mt, tn);
     rc = rc ? rc : g->alloc(&g->vt, tn);
     rc = rc ? rc : g->alloc(&g->t16, tn);

@@ -132,6 +132,17 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// 32 columns, load and wait in one block: the compiler cannot place a spill or a
+// copy of the destination registers between the two.
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+}
+
 // The same without the wait, so several loads share one tcgen05.wait::ld.
 __device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t* r) {
     asm volatile(
@@ -154,6 +165,31 @@ __device__ __forceinline__ void group_sync(uint32_t grp) {
         case 5: asm volatile("bar.sync 6, 128;" ::: "memory"); break;
         default: asm volatile("bar.sync 7, 128;" ::: "memory"); break;
     }
+}
+
+// An operand in the core-matrix layout as one MMA step reads it: K-major (its
+// rows are M or N, its columns K), or transposed (its rows are K, its columns
+// M or N, the "MN-major" form of the same core matrices). `cols` is the
+// operand's stored row length. Core matrices 8 columns apart are 128 bytes
+// apart and those 8 rows apart cols * 16; the descriptor's stride offset steps
+// along M or N and its leading offset along K.
+struct UmmaOperand {
+    uint32_t saddr, lbo, sbo, kstep;
+    uint32_t trans;
+};
+__device__ __forceinline__ UmmaOperand umma_k_major(uint32_t saddr, uint32_t cols) {
+    return {saddr, 128u, cols * 16u, 256u, 0u};
+}
+__device__ __forceinline__ UmmaOperand umma_transposed(uint32_t saddr, uint32_t cols) {
+    return {saddr, cols * 16u, 128u, cols * 32u, 1u};
+}
+// Issue D[128][N] = A B over K in either operand form (one thread issues).
+__device__ __forceinline__ void tc_gemm_issue_ops(uint32_t d_tmem, const UmmaOperand& A, const UmmaOperand& B, int N,
+                                                  int K) {
+    const uint32_t idesc = umma_idesc_bf16_f32(128, N) | (A.trans << 15) | (B.trans << 16);
+    for (int ks = 0; ks < K / 16; ks++)
+        tc_mma_bf16(d_tmem, umma_smem_desc(A.saddr + ks * A.kstep, A.lbo, A.sbo),
+                    umma_smem_desc(B.saddr + ks * B.kstep, B.lbo, B.sbo), idesc, ks > 0 ? 1u : 0u);
 }
 
 // Issue D = A * B^T for a 128-row tile (thread 0 of the CTA issues).
