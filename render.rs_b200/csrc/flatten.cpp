@@ -106,7 +106,10 @@ struct BinBvh {
 // primitives' boxes and centroids are partitioned in place with their
 // indices (the reference's swap partition, same order), so every pass over a
 // node's range reads memory sequentially.
-BinBvh build_binary(const std::vector<Box>& bounds) {
+// max_leaf: leaves of at most that many primitives (up to four times as many
+// when SAH prefers one); 1 for the TLAS, whose leaves hold one item each and
+// which takes every finite SAH split (bvh_build.cu has the reason).
+BinBvh build_binary(const std::vector<Box>& bounds, size_t max_leaf = 4) {
 // Build-time options. 32 bins, or SAH over all three axes, traced the
 // 1M-triangle cloud within 2% of the reference's rule (16 bins, widest axis)
 // and took 6-28% longer to build, so the reference's rule is the default.
@@ -116,7 +119,7 @@ BinBvh build_binary(const std::vector<Box>& bounds) {
 #ifndef RT_SAH_ALL_AXES
 #define RT_SAH_ALL_AXES 0   // 0: the widest centroid axis only (the reference's rule)
 #endif
-    const int BINS = RT_SAH_BINS, MAX_LEAF = 4;
+    const int BINS = RT_SAH_BINS;
     BinBvh t;
     size_t n = bounds.size();
     t.order.resize(n);
@@ -197,7 +200,7 @@ BinBvh build_binary(const std::vector<Box>& bounds) {
             nodes[j.node].first = (uint32_t)j.start;
             nodes[j.node].count = (uint32_t)j.count;
         };
-        if (j.count <= (size_t)MAX_LEAF) {
+        if (j.count <= max_leaf) {
             make_leaf();
             return false;
         }
@@ -272,7 +275,7 @@ BinBvh build_binary(const std::vector<Box>& bounds) {
             }
             const double amin = cb.lo[axis], aext = ext[axis];
             double leaf_cost = b.area() * (double)j.count;
-            if (std::isfinite(best) && best < leaf_cost) {
+            if (std::isfinite(best) && (best < leaf_cost || max_leaf == 1)) {
                 double boundary = amin + aext * (double)(best_bin + 1) / (double)BINS;
                 size_t m = 0;
                 if (wide_node) {
@@ -312,7 +315,7 @@ BinBvh build_binary(const std::vector<Box>& bounds) {
                     }
                 }
                 if (m > 0 && m < j.count) split = j.start + m;
-            } else if (j.count <= (size_t)MAX_LEAF * 4) {
+            } else if (j.count <= max_leaf * 4 && max_leaf > 1) {
                 make_leaf();
                 return false;
             }
@@ -1502,7 +1505,7 @@ bool flatten_scene(const rt_scene_desc* d, HostScene* out, std::string* err, boo
                         ib[i].hi[a] = boxes[6 * i + 3 + a];
                     }
             });
-            BinBvh tl = build_binary(ib);
+            BinBvh tl = build_binary(ib, 1);
             Collapser col{tl, H.nodes, 0};
             H.scalars.tlas_root = col.emit(0);
             col.finish();

@@ -736,7 +736,7 @@ __device__ __forceinline__ void ray_pump(const DevScene& S, uint32_t n, uint32_t
                     // One step: enter a parked instance leaf, or pop; then
                     // test the node that is current, if any.
                     if (RT_INST_IN_NODE_PHASE && ps.pending && !ps.ts.in_inst)
-                        done_now = op_leaf<ANY, MOT>(S, ps, st, err);
+                        done_now = op_leaf<ANY, MOT>(S, ps, st);
                     else if (ps.need_pop)
                         done_now = !op_pop(ps, st);
                     if (!done_now && ps.pending == 0 && !ps.need_pop) done_now = op_node<ANY>(S, ps, st, err);
@@ -752,7 +752,7 @@ __device__ __forceinline__ void ray_pump(const DevScene& S, uint32_t n, uint32_t
         // Leaf phase: instance leaves (TLAS) per lane, then the warp's
         // triangle leaves together (leaf_coop).
         bool done_now = false;
-        if (active && ps.pending && !ps.ts.in_inst) done_now = op_leaf<ANY, MOT>(S, ps, st, err);
+        if (active && ps.pending && !ps.ts.in_inst) done_now = op_leaf<ANY, MOT>(S, ps, st);
         const bool tri_leaf = active && !done_now && ps.pending && ps.ts.in_inst;
         if (__any_sync(0xFFFFFFFFu, tri_leaf))
             done_now |= leaf_coop<ANY, TRANSMIT, PRES, CURV, MOT>(S, ps, tri_leaf, leaf, ray_seed);

@@ -387,26 +387,16 @@ struct TravStack {
     uint2* sh;       // this thread's column: entry k at sh[k * stride]
     int stride;
     int sp;
-    bool overflow;
     uint2 spill[RT_SPILL];
 
     __device__ __forceinline__ void init(uint2* col, int stride_) {
         sh = col;
         stride = stride_;
         sp = 0;
-        overflow = false;
     }
     __device__ __forceinline__ void put(int i, uint32_t ref, uint32_t t) {
         if (i < RT_SH_STACK) sh[i * stride] = make_uint2(ref, t);
         else spill[i - RT_SH_STACK] = make_uint2(ref, t);
-    }
-    __device__ __forceinline__ void push(uint32_t ref, float t) {
-        if (sp >= RT_SH_STACK + RT_SPILL) {
-            overflow = true;
-            return;
-        }
-        put(sp, ref, __float_as_uint(t));
-        sp++;
     }
     __device__ __forceinline__ uint2 pop() {
         sp--;
@@ -458,7 +448,6 @@ __device__ __forceinline__ bool trav_begin(const DevScene& S, TravState& ts, Tra
     ts.steps = 0;
     ts.trans = 1.0f;
     st.sp = 0;
-    st.overflow = false;
     if (S.tlas_root == 0xFFFFFFFFu) return false;
     ray_boxes(ts.r, o, d);  // no triangles at the top level
     ts.cur = S.tlas_root;
@@ -587,22 +576,16 @@ __device__ __forceinline__ bool op_node(const DevScene& S, PhaseState& ps, TravS
     return false;
 }
 
-// Returns true when the query is over (any-hit found, or a fatal condition).
-// MOT: instances and triangles are placed at the ray's shutter time.
+// Returns true when the query is over (any-hit found). MOT: instances and triangles are placed at the ray's shutter time.
 template <bool ANY, bool MOT = false>
-__device__ __forceinline__ bool op_leaf(const DevScene& S, PhaseState& ps, TravStack& st, uint32_t* err) {
+__device__ __forceinline__ bool op_leaf(const DevScene& S, PhaseState& ps, TravStack& st) {
     TravState& ts = ps.ts;
     const uint32_t leaf = ps.pending;
     ps.pending = 0;
     uint32_t first = leaf & LEAF_FIRST_MASK;
     uint32_t count = ((leaf >> 27) & 15u) + 1u;
     if (!ts.in_inst) {
-        for (uint32_t k = count - 1; k >= 1; k--) st.push(make_leaf_ref(first + k, 1), 0.0f);
-        if (st.overflow) {
-            atomicOr(err, RT_DEVERR_STACK);
-            return true;
-        }
-        // TLAS item: (instance, child of its BLAS root); the child is a
+        // The leaf's one TLAS item: (instance, child of its BLAS root); the child is a
         // node to descend from or a triangle leaf tested in this leaf phase.
         const uint2 item = __ldg(S.items + first);
         const uint32_t inst = item.x, root = item.y;
