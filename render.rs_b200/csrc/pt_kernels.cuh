@@ -125,14 +125,12 @@ struct PtConsts {
 #define FL_DEPTH_SHIFT 16
 
 #define RT_RAY_OFFSET 1e-4f
-// Traversal kernels are latency-bound at a few warps per SM: asking the
-// register allocator for 5 resident 128-thread blocks (at most 102 registers,
-// no spills) raised closest hit from 219 to 246 Mrays/s on the 1M-triangle
-// cloud; 6 blocks spills and no longer fits the 39 KB of shared memory a
-// block holds with the 32-entry stack.
-#ifndef RT_TRAV_MIN_BLOCKS
+// Resident 128-thread blocks per SM the traversal kernels ask for. They are
+// bound by latency and issue at a few warps per scheduler, so blocks count as
+// long as nothing spills: closest-hit and any-hit kernels without cutouts,
+// quadrics or motion fit 80 registers (six blocks), the others 96 (five).
 #define RT_TRAV_MIN_BLOCKS 5
-#endif
+#define RT_TRAV_PLAIN_BLOCKS 6
 #define RT_MAX_PRESENCE_SKIPS 16u
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
@@ -1026,9 +1024,10 @@ __device__ __forceinline__ float light_pdf_sa(const DevLight& L, float3 origin, 
     return 0.0f;
 }
 
-#ifndef RT_SHADE_MIN_BLOCKS
-#define RT_SHADE_MIN_BLOCKS 1
-#endif
+// Four resident blocks: 124 registers without spills, where the compiler's own
+// choice of 140 left three (materials 1080p x 6 spp: 4.8 -> 4.0 ms of shading;
+// five spill and take 4.3).
+#define RT_SHADE_MIN_BLOCKS 4
 // PAT: the scene has patterns (ray cones tracked, patterned materials
 // resolved per hit). The plain instance keeps its material reads on the
 // global material table and the register count of a kernel without them.
@@ -1513,8 +1512,8 @@ __global__ void __launch_bounds__(128, RT_SHADE_MIN_BLOCKS) k_shade(DevScene S, 
 }
 
 // ---- shadow -------------------------------------------------------------------------------
-template <int BLOCK, bool QUAD = false, bool MOT = false>
-__global__ void __launch_bounds__(BLOCK, RT_TRAV_MIN_BLOCKS) k_shadow(DevScene S, Paths P, PtConsts C) {
+template <int BLOCK, bool TRANS, bool QUAD = false, bool MOT = false>
+__global__ void __launch_bounds__(BLOCK, TRANS || QUAD || MOT ? RT_TRAV_MIN_BLOCKS : RT_TRAV_PLAIN_BLOCKS) k_shadow(DevScene S, Paths P, PtConsts C) {
     __shared__ uint2 stack_sh[RT_SH_STACK * BLOCK];
     __shared__ LeafShared leaf_sh[BLOCK / 32];
     TravStack st;
@@ -1530,7 +1529,7 @@ __global__ void __launch_bounds__(BLOCK, RT_TRAV_MIN_BLOCKS) k_shadow(DevScene S
             P.aux_d[slot] = make_float4(a.x + c.x * vis, a.y + c.y * vis, a.z + c.z * vis, a.w);
         }
     };
-    if (!S.any_presence) {
+    if constexpr (!TRANS) {
         // Opaque scenes: one any-hit query per shadow ray, through the pump.
         uint32_t slot = 0;
         bool qblock = false;  // a quadric blocks this lane's shadow ray
@@ -1556,36 +1555,35 @@ __global__ void __launch_bounds__(BLOCK, RT_TRAV_MIN_BLOCKS) k_shadow(DevScene S
         };
         ray_pump<true, false, false, QUAD, MOT>(S, n, &P.cnt[CNT_FETCH_SH], P.err, st, leaf_sh[threadIdx.x >> 5], load,
                                                 finish);
-        if (rays) atomicAdd(&P.stats[1], rays);
-        return;
+    } else {
+        // Scenes with presence cutouts: transmittance queries through the pump
+        // (traverse.cuh: one traversal per shadow ray, cutouts attenuate, opaque
+        // surfaces block).
+        uint32_t slot = 0;
+        float qvis = 1.0f;  // transmittance of this lane's shadow ray through the quadrics
+        auto load = [&](uint32_t j, float3& o, float3& d, float& tmax, uint64_t& seed, float& time) {
+            slot = P.q_sh[j];
+            float4 o4 = P.sh_o[slot], d4 = P.sh_d[slot];
+            o = xyz(o4);
+            d = xyz(d4);
+            tmax = d4.w;
+            if (MOT) time = P.time[slot];
+            qvis = 1.0f;
+            if (QUAD) {
+                const float dl = fmaxf(length(d), 1e-30f);
+                qvis = quadrics_transmittance(S, o, d / dl, tmax * dl);
+                if (qvis == 0.0f) tmax = -1.0f;  // nothing left for the BVH to find
+            }
+        };
+        auto finish = [&](bool done, uint32_t, const TravState& ts) {
+            if (!done) return;
+            rays++;
+            const float vis = ts.trans * qvis;
+            if (vis > 0.0f) add(slot, vis);
+        };
+        ray_pump<true, true, false, QUAD, MOT>(S, n, &P.cnt[CNT_FETCH_SH], P.err, st, leaf_sh[threadIdx.x >> 5], load,
+                                               finish);
     }
-    // Scenes with presence cutouts: transmittance queries through the pump
-    // (traverse.cuh: one traversal per shadow ray, cutouts attenuate, opaque
-    // surfaces block).
-    uint32_t slot = 0;
-    float qvis = 1.0f;  // transmittance of this lane's shadow ray through the quadrics
-    auto load = [&](uint32_t j, float3& o, float3& d, float& tmax, uint64_t& seed, float& time) {
-        slot = P.q_sh[j];
-        float4 o4 = P.sh_o[slot], d4 = P.sh_d[slot];
-        o = xyz(o4);
-        d = xyz(d4);
-        tmax = d4.w;
-        if (MOT) time = P.time[slot];
-        qvis = 1.0f;
-        if (QUAD) {
-            const float dl = fmaxf(length(d), 1e-30f);
-            qvis = quadrics_transmittance(S, o, d / dl, tmax * dl);
-            if (qvis == 0.0f) tmax = -1.0f;  // nothing left for the BVH to find
-        }
-    };
-    auto finish = [&](bool done, uint32_t, const TravState& ts) {
-        if (!done) return;
-        rays++;
-        const float vis = ts.trans * qvis;
-        if (vis > 0.0f) add(slot, vis);
-    };
-    ray_pump<true, true, false, QUAD, MOT>(S, n, &P.cnt[CNT_FETCH_SH], P.err, st, leaf_sh[threadIdx.x >> 5], load,
-                                           finish);
     if (rays) atomicAdd(&P.stats[1], rays);
 }
 
@@ -1897,7 +1895,7 @@ __global__ void k_resolve(const double* __restrict__ accum, float* __restrict__ 
 
 // ---- ray batch (rt_intersect_batch) ------------------------------------------------------
 template <int BLOCK, bool ANY, bool QUAD = false>
-__global__ void __launch_bounds__(BLOCK, RT_TRAV_MIN_BLOCKS) k_intersect(DevScene S, const float4* __restrict__ org,
+__global__ void __launch_bounds__(BLOCK, QUAD ? RT_TRAV_MIN_BLOCKS : RT_TRAV_PLAIN_BLOCKS) k_intersect(DevScene S, const float4* __restrict__ org,
                                                      const float4* __restrict__ dir, uint64_t n, uint32_t* prim,
                                                      uint32_t* inst, float* tout, uint32_t* fetch, uint32_t* err) {
     __shared__ uint2 stack_sh[RT_SH_STACK * BLOCK];

@@ -170,7 +170,8 @@ struct rt_session {
     rt_stats last{};
     cudaEvent_t ev[8] = {};
     std::vector<cudaEvent_t> evpool;
-    int trav_grid = 148 * 4;      // resident blocks of the traversal kernels
+    int trav_grid = 148 * RT_TRAV_MIN_BLOCKS;     // resident blocks of the traversal kernels
+    int plain_grid = 148 * RT_TRAV_PLAIN_BLOCKS;  // and of their plain variants
 
     template <class T>
     int alloc(T** p, size_t count) {
@@ -229,9 +230,10 @@ struct rt_session {
 static bool extra_geometry(const rt_session* s) { return s->S.n_quadrics > 0 || s->S.any_curves; }
 
 // The ray-batch kernel variant for the query and the scene.
-static void launch_intersect(rt_session* s, int any_hit, int grid, cudaStream_t st, const float4* o, const float4* d,
+static void launch_intersect(rt_session* s, int any_hit, cudaStream_t st, const float4* o, const float4* d,
                              uint64_t n, uint32_t* prim, uint32_t* inst, float* t, uint32_t* fetch, uint32_t* err) {
     const bool quad = extra_geometry(s);
+    const int grid = quad ? s->trav_grid : s->plain_grid;
     if (any_hit && quad)
         k_intersect<TRAV_BLOCK, true, true><<<grid, TRAV_BLOCK, 0, st>>>(s->S, o, d, n, prim, inst, t, fetch, err);
     else if (any_hit)
@@ -240,6 +242,15 @@ static void launch_intersect(rt_session* s, int any_hit, int grid, cudaStream_t 
         k_intersect<TRAV_BLOCK, false, true><<<grid, TRAV_BLOCK, 0, st>>>(s->S, o, d, n, prim, inst, t, fetch, err);
     else
         k_intersect<TRAV_BLOCK, false><<<grid, TRAV_BLOCK, 0, st>>>(s->S, o, d, n, prim, inst, t, fetch, err);
+}
+
+// The shadow kernel variant: TRANS attenuates through cutouts.
+template <bool TRANS>
+static void launch_shadow(rt_session* s, const Paths& P, const PtConsts& C, cudaStream_t st) {
+    const int grid = TRANS || s->S.motion || extra_geometry(s) ? s->trav_grid : s->plain_grid;
+    if (s->S.motion) k_shadow<TRAV_BLOCK, TRANS, true, true><<<grid, TRAV_BLOCK, 0, st>>>(s->S, P, C);
+    else if (extra_geometry(s)) k_shadow<TRAV_BLOCK, TRANS, true><<<grid, TRAV_BLOCK, 0, st>>>(s->S, P, C);
+    else k_shadow<TRAV_BLOCK, TRANS><<<grid, TRAV_BLOCK, 0, st>>>(s->S, P, C);
 }
 
 extern "C" {
@@ -276,6 +287,9 @@ int rt_session_create(const rt_scene_desc* scene, const rt_params* params, rt_se
         int nb = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_extend<TRAV_BLOCK, false>, TRAV_BLOCK, 0);
         s->trav_grid = s->sm_count * std::max(nb, 1);
+        nb = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_intersect<TRAV_BLOCK, false>, TRAV_BLOCK, 0);
+        s->plain_grid = s->sm_count * std::max(nb, 1);
     }
     cudaError_t ce = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
     if (ce != cudaSuccess) {
@@ -648,9 +662,10 @@ int rt_render_samples(rt_session* s, uint32_t sample_start, uint32_t count) {
             else if (med) k_shadow_walk<TRAV_BLOCK><<<trav_grid, TRAV_BLOCK, 0, st>>>(s->S, P, C);
             else if (s->S.presence_pat)
                 k_shadow_walk<TRAV_BLOCK, false, true><<<trav_grid, TRAV_BLOCK, 0, st>>>(s->S, P, C);
-            else if (mot) k_shadow<TRAV_BLOCK, true, true><<<trav_grid, TRAV_BLOCK, 0, st>>>(s->S, P, C);
-            else if (quad) k_shadow<TRAV_BLOCK, true><<<trav_grid, TRAV_BLOCK, 0, st>>>(s->S, P, C);
-            else k_shadow<TRAV_BLOCK><<<trav_grid, TRAV_BLOCK, 0, st>>>(s->S, P, C);
+            else if (s->S.any_presence)
+                launch_shadow<true>(s, P, C, st);
+            else
+                launch_shadow<false>(s, P, C, st);
             CUDA_TRY(cudaEventRecord(s->evpool[ei + 3], st));
             k_wave_prep<<<1, 32, 0, st>>>(P.cnt);
             launches += 4;
@@ -874,8 +889,7 @@ int rt_intersect_batch_device(rt_session* s, const float* rays, uint64_t n, int 
     CUDA_TRY(cudaMemsetAsync(s->fetch, 0, 4, st));
     const float4* o = (const float4*)rays;
     const float4* d = o + n;
-    int grid = s->trav_grid;
-    launch_intersect(s, any_hit, grid, st, o, d, n, prim, inst, t, s->fetch, s->err);
+    launch_intersect(s, any_hit, st, o, d, n, prim, inst, t, s->fetch, s->err);
     CUDA_TRY(cudaGetLastError());
     return RT_OK;
 }
@@ -973,7 +987,7 @@ extern "C" int rt_intersect_batch_noalloc(rt_session* s, const float* rays, uint
     CUDA_TRY(cudaMemsetAsync(d_err, 0, 4, st));
     const float4* o = (const float4*)d_rays;
     const float4* d = o + n;
-    launch_intersect(s, any_hit, s->trav_grid, st, o, d, n, d_prim, d_inst, d_t, d_fetch, d_err);
+    launch_intersect(s, any_hit, st, o, d, n, d_prim, d_inst, d_t, d_fetch, d_err);
     CUDA_TRY(cudaGetLastError());
     uint32_t e = 0;
     CUDA_TRY(cudaMemcpyAsync(prim, d_prim, 4 * n, cudaMemcpyDeviceToHost, st));

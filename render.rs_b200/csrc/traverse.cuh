@@ -427,6 +427,7 @@ struct TravState {
     uint32_t steps;
     int inst_sp;
     bool in_inst, found;
+    bool sheared;      // the ray's shear for this instance is made
     float trans;       // shadow transmittance (TRANSMIT queries)
     float time;        // shutter time of the ray (motion blur; 0 in static scenes)
 };
@@ -593,7 +594,7 @@ __device__ __forceinline__ bool op_leaf(const DevScene& S, PhaseState& ps, TravS
         float4 x0, x1, x2;
         inst_rows<MOT>(S, inst, ts.time, x0, x1, x2);
         ray_boxes(ts.r, xf_point(x0, x1, x2, ts.o), xf_vec(x0, x1, x2, ts.d));
-        ray_shear(ts.r);
+        ts.sheared = false;
         ts.in_inst = true;
         ts.inst_sp = st.sp;
         ts.cur = root;
@@ -601,6 +602,10 @@ __device__ __forceinline__ bool op_leaf(const DevScene& S, PhaseState& ps, TravS
         if (root & REF_LEAF) ps.pending = root;
         else ps.need_pop = false;
         return false;
+    }
+    if (!ts.sheared) {
+        ray_shear(ts.r);
+        ts.sheared = true;
     }
     for (uint32_t k = 0; k < count; k++) {
         float4 a, b, c;
@@ -690,6 +695,12 @@ __device__ __forceinline__ bool leaf_coop(const DevScene& S, PhaseState& ps, boo
         count = ((ps.pending >> 27) & 15u) + 1u;
         ps.pending = 0;
         ps.need_pop = true;
+        // The shear is made at the first triangle leaf after entering an
+        // instance: many entered instances are left without one.
+        if (!ts.sheared) {
+            ray_shear(ts.r);
+            ts.sheared = true;
+        }
     }
     uint32_t incl = count;
 #pragma unroll
@@ -700,7 +711,7 @@ __device__ __forceinline__ bool leaf_coop(const DevScene& S, PhaseState& ps, boo
     const uint32_t excl = incl - count, total = __shfl_sync(0xFFFFFFFFu, incl, 31);
     for (uint32_t k = 0; k < count; k++) L.item[excl + k] = (uint16_t)((lane << 4) | k);
     L.key[lane] = ~0ull;
-    L.trans[lane] = 1.0f;
+    if (TRANSMIT) L.trans[lane] = 1.0f;
     // TRANSMIT / PRES: the presence of the material of this lane's instance.
     const float pres_own =
         ((TRANSMIT || PRES) && mine) ? __ldg(&S.materials[__ldg(&S.inst[ts.cur_inst].z)].presence) : 1.0f;
@@ -731,7 +742,7 @@ __device__ __forceinline__ bool leaf_coop(const DevScene& S, PhaseState& ps, boo
             r.d.y = __shfl_sync(0xFFFFFFFFu, ts.r.d.y, owner);
             r.d.z = __shfl_sync(0xFFFFFFFFu, ts.r.d.z, owner);
         }
-        const float pres = __shfl_sync(0xFFFFFFFFu, pres_own, owner);
+        const float pres = (TRANSMIT || PRES) ? __shfl_sync(0xFFFFFFFFu, pres_own, owner) : 1.0f;
         const float tm = MOT ? __shfl_sync(0xFFFFFFFFu, ts.time, owner) : 0.0f;
         uint64_t seed = 0;
         uint32_t inst_o = 0;
@@ -748,7 +759,7 @@ __device__ __forceinline__ bool leaf_coop(const DevScene& S, PhaseState& ps, boo
             // Cull with the best hit so far, keeping hits at equal t (they
             // compete on the triangle index).
             if (!TRANSMIT && best != ~0ull)
-                tmax = fminf(tmax, nextafterf(__uint_as_float((uint32_t)(best >> 32)), INFINITY));
+                tmax = fminf(tmax, __uint_as_float((uint32_t)(best >> 32) + 1u));  // the next float up (t > 0, finite)
             const uint32_t tri = f + (it & 15u);
             float4 a, b, c;
             tri_at<MOT>(S, tri, tm, a, b, c);
