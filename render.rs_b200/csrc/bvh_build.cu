@@ -41,7 +41,9 @@ constexpr int BINS = 16;
 // transform, and a node or triangles to fetch) where the item's own box among
 // its parent's eight costs 20 instructions: with leaves of up to four,
 // 1.5M any-hit rays into 1,000 instances 2.07 ms, now 1.52; forest 60 -> 47 ms.
+// A mesh of up to RT_SMALL_MESH triangles takes RT_SMALL_MESH_LEAF (rt_internal.h).
 constexpr uint32_t MAX_LEAF = 4;
+
 constexpr uint32_t SAH_LEAF_MAX = 16;
 constexpr uint32_t SMALL = 256;        // subtrees of at most this many primitives: one warp each
 constexpr uint32_t CHUNK = 2048;       // primitives per block in the level passes
@@ -623,7 +625,8 @@ __global__ void k_clear_acc(ChildArgs C, uint32_t n) {
 // entries.
 __global__ void __launch_bounds__(32 * SMALL_WARPS)
     k_subtrees(const Job* __restrict__ small, const uint32_t* n_small_p, BPrim* P0, BPrim* P1, BNode* nodes,
-               uint32_t* node_counter, uint32_t node_cap, uint32_t* err, uint32_t max_leaf) {
+               uint32_t* node_counter, uint32_t node_cap, uint32_t* err, uint32_t leaf_large, uint32_t leaf_small,
+               uint32_t n_roots) {
     __shared__ uint32_t bins_sh[SMALL_WARPS][BINS * 7];
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const uint32_t w = blockIdx.x * SMALL_WARPS + wib;
@@ -633,6 +636,8 @@ __global__ void __launch_bounds__(32 * SMALL_WARPS)
     Job stack[STACK];
     int sp = 0;
     stack[sp++] = small[w];
+    // The first n_roots subtrees are whole trees, the rest parts of larger ones.
+    const uint32_t max_leaf = w < n_roots && stack[0].count <= RT_SMALL_MESH ? leaf_small : leaf_large;
     while (sp > 0) {
         const Job J = stack[--sp];
         const BPrim* src = J.parity ? P1 : P0;
@@ -1145,7 +1150,8 @@ std::string berr_text(uint32_t e) {
 // On return P0 holds the primitives in leaf order.
 int build_binary_device(Scratch& D, BPrim* P0, BPrim* P1, uint32_t n,
                         const std::vector<std::pair<uint32_t, uint32_t>>& roots, uint32_t* d_err, BNode** nodes_out,
-                        uint32_t* n_nodes_out, cudaStream_t st, std::string* err, uint32_t max_leaf) {
+                        uint32_t* n_nodes_out, cudaStream_t st, std::string* err, uint32_t max_leaf,
+                        uint32_t small_leaf) {
     const uint32_t R = (uint32_t)roots.size();
     const uint64_t node_cap = 2ull * n + R + 2;
     const uint32_t J_cap = n / (SMALL + 1) + 2;
@@ -1253,7 +1259,8 @@ int build_binary_device(Scratch& D, BPrim* P0, BPrim* P1, uint32_t n,
     }
     if (host_ctr[3]) {
         k_subtrees<<<blocks_for(host_ctr[3], SMALL_WARPS), 32 * SMALL_WARPS, 0, st>>>(
-            small, &counters[3], P0, P1, nodes, &counters[0], C.node_cap, d_err, max_leaf);
+            small, &counters[3], P0, P1, nodes, &counters[0], C.node_cap, d_err, max_leaf, small_leaf,
+            (uint32_t)sj.size());
     }
     uint32_t e = 0;
     BV_TRY(cudaMemcpyAsync(host_ctr, counters, sizeof(host_ctr), cudaMemcpyDeviceToHost, st));
@@ -1429,7 +1436,8 @@ int device_build_scene(const rt_scene_desc* d, HostScene* H, DeviceBvh* out, cud
             return RT_ERR_INVALID;
         }
         uint32_t n_bnodes = 0;
-        rc = build_binary_device(D, P0, P1, (uint32_t)N, roots, d_err, &bnodes, &n_bnodes, st, err, MAX_LEAF);
+        rc = build_binary_device(D, P0, P1, (uint32_t)N, roots, d_err, &bnodes, &n_bnodes, st, err, MAX_LEAF,
+                                 small_mesh_leaves(d) ? RT_SMALL_MESH_LEAF : MAX_LEAF);
         if (rc) return rc;
         H->binary_blas_nodes = n_bnodes;
         rc = wide_structure(D, bnodes, n_bnodes, (uint32_t)roots.size(), d_err, &bw, st, err);
@@ -1570,7 +1578,7 @@ int device_build_scene(const rt_scene_desc* d, HostScene* H, DeviceBvh* out, cud
         }
         if (NIT) {
             uint32_t n_tnodes = 0;
-            rc = build_binary_device(D, Q0, Q1, NIT, {{0u, NIT}}, d_err, &tnodes, &n_tnodes, st, err, 1);
+            rc = build_binary_device(D, Q0, Q1, NIT, {{0u, NIT}}, d_err, &tnodes, &n_tnodes, st, err, 1, 1);
             if (rc) return rc;
             rc = wide_structure(D, tnodes, n_tnodes, 1, d_err, &tw, st, err);
             if (rc) return rc;

@@ -106,8 +106,8 @@ struct BinBvh {
 // primitives' boxes and centroids are partitioned in place with their
 // indices (the reference's swap partition, same order), so every pass over a
 // node's range reads memory sequentially.
-// max_leaf: leaves of at most that many primitives (up to four times as many
-// when SAH prefers one); 1 for the TLAS, whose leaves hold one item each and
+// max_leaf: leaves of at most that many primitives (up to 16 when SAH prefers
+// one); 1 for the TLAS, whose leaves hold one item each and
 // which takes every finite SAH split (bvh_build.cu has the reason).
 BinBvh build_binary(const std::vector<Box>& bounds, size_t max_leaf = 4) {
 // Build-time options. 32 bins, or SAH over all three axes, traced the
@@ -315,7 +315,7 @@ BinBvh build_binary(const std::vector<Box>& bounds, size_t max_leaf = 4) {
                     }
                 }
                 if (m > 0 && m < j.count) split = j.start + m;
-            } else if (j.count <= max_leaf * 4 && max_leaf > 1) {
+            } else if (j.count <= 16 && max_leaf > 1) {
                 make_leaf();
                 return false;
             }
@@ -1203,6 +1203,15 @@ bool flatten_quadrics(const rt_scene_desc* d, HostScene& H, std::string* err) {
     return true;
 }
 
+bool small_mesh_leaves(const rt_scene_desc* d) {
+    for (uint32_t m = 0; m < d->n_materials; m++)
+        if (!(d->materials[m].presence >= 1.0)) return false;
+    for (uint32_t b = 0; b < d->n_bindings; b++)
+        if (d->bindings[b].field == RT_FIELD_PRESENCE) return false;
+    return true;
+}
+
+
 bool flatten_scene(const rt_scene_desc* d, HostScene* out, std::string* err, bool build_bvh) {
     HostScene& H = *out;
     if (!d) {
@@ -1275,6 +1284,7 @@ bool flatten_scene(const rt_scene_desc* d, HostScene* out, std::string* err, boo
     std::vector<std::vector<RootChild>> root_children(n_geom), grand_children(n_geom);
     H.meshes.resize(n_geom);
     uint64_t tri_total = 0;
+    const bool small_leaves = small_mesh_leaves(d);
     for (uint32_t m = 0; m < d->n_meshes; m++) tri_total += d->meshes[m].n_triangles;
     for (uint32_t k = 0; k < d->n_curves; k++) tri_total += d->curves[k].n_segments;
     if (tri_total >= (1ull << 27)) {
@@ -1390,7 +1400,8 @@ bool flatten_scene(const rt_scene_desc* d, HostScene* out, std::string* err, boo
             *err = "mesh " + std::to_string(m) + " has a non-finite vertex";
             return false;
         }
-        BinBvh bin = build_binary(tb);
+        const bool small = small_leaves && md.n_triangles <= RT_SMALL_MESH;
+        BinBvh bin = build_binary(tb, small ? RT_SMALL_MESH_LEAF : 4);
         H.binary_blas_nodes += bin.nodes.size();
         const size_t tri_off = H.tris.size();
         H.tris.resize(tri_off + 3ull * md.n_triangles);

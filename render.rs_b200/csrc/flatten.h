@@ -61,6 +61,10 @@ struct HostScene {
 // their triangle ranges but no BLAS root, and vertex data is not validated.
 bool flatten_scene(const rt_scene_desc* desc, HostScene* out, std::string* err, bool build_bvh = true);
 
+// Leaf size of a mesh (rt_internal.h): small meshes of scenes without presence
+// cutouts, constant or bound to a pattern, get smaller leaves.
+bool small_mesh_leaves(const rt_scene_desc* d);
+
 // One child of a mesh's BLAS root: its exact box and its reference (wide
 // node index or leaf reference).
 struct RootChild {

@@ -55,3 +55,32 @@ def test_builders_agree_and_match_oracle(n, spread):
     both = hit & (a[0] != 0xFFFFFFFF)
     assert (np.abs(a[2][both] - ot[both]) <= 1e-4 * (1.0 + ot[both])).mean() > 0.999
     assert (a[3] == hit).mean() > 0.999
+
+
+@pytest.mark.parametrize("presence", [1.0, 0.5])
+@pytest.mark.parametrize("tris", [1, 2, 3, 5, 17, 63, 64, 65, 300])
+def test_small_meshes_build_alike(tris, presence):
+    """Meshes around the small-mesh limit (leaves of two instead of four, four in scenes with cutouts)."""
+    s = Scene(8, 8)
+    mat = s.add_material(matte((0.5, 0.5, 0.5), presence=presence))
+    pos, idx = scenes.triangle_cloud_mesh(tris, seed=tris)
+    s.add_instance(s.add_mesh(pos * 4.0, idx), mat)
+    s.add_instance(s.add_mesh(*scenes.unit_cube()), mat, affine(np.eye(3), (3.0, 0.0, 0.0)))
+    rays = scenes.triangle_cloud_rays(4096, seed=7)
+    rays[0, :, :3] *= 3.0
+    target = pos.reshape(-1, 3, 3)[np.arange(4096) % tris].mean(1) * 4.0
+    d = target - rays[0, :, :3]
+    rays[1, :, :3] = d / np.linalg.norm(d, axis=1, keepdims=True)
+    got = {}
+    for build in ("device", "host"):
+        with PtSession(s, abi.make_params(max_depth=4, max_paths=64, bvh_build=build)) as g:
+            st = g.stats()
+            got[build] = g.intersect(rays) + (st["blas_nodes"], st["tlas_nodes"])
+    a, b = got["device"], got["host"]
+    assert a[3:] == b[3:]
+    assert np.array_equal(a[2], b[2])
+    op, _, ot, _ = oracle.OracleScene(s).intersect(rays)
+    hit = op != 0xFFFFFFFF
+    assert hit.sum() > 2000 and ((a[0] != 0xFFFFFFFF) == hit).mean() > 0.999
+    both = hit & (a[0] != 0xFFFFFFFF)
+    assert (np.abs(a[2][both] - ot[both]) <= 1e-4 * (1.0 + ot[both])).mean() > 0.999
