@@ -236,7 +236,7 @@ __device__ __forceinline__ bool trace_closest(const DevScene& S, TravStack& st, 
                 if (op_leaf<false, MOT>(S, ps, st)) break;
             } else if (ps.need_pop) {
                 if (!op_pop(ps, st)) break;
-            } else if (op_node<false>(S, ps, st, err)) {
+            } else if (op_node<true>(S, ps, st, err)) {
                 break;
             }
         }

@@ -737,11 +737,11 @@ __device__ __forceinline__ void ray_pump(const DevScene& S, uint32_t n, uint32_t
                         done_now = op_leaf<ANY, MOT>(S, ps, st);
                     else if (ps.need_pop)
                         done_now = !op_pop(ps, st);
-                    if (!done_now && ps.pending == 0 && !ps.need_pop) done_now = op_node<ANY>(S, ps, st, err);
+                    if (!done_now && ps.pending == 0 && !ps.need_pop) done_now = op_node<!TRANSMIT>(S, ps, st, err);
                 } else if (ps.need_pop) {
                     done_now = !op_pop(ps, st);
                 } else {
-                    done_now = op_node<ANY>(S, ps, st, err);
+                    done_now = op_node<!TRANSMIT>(S, ps, st, err);
                 }
             }
             fin |= done_now;

@@ -502,7 +502,12 @@ __device__ __forceinline__ bool op_pop(PhaseState& ps, TravStack& st) {
 }
 
 // Returns true on a fatal condition (stack overflow): the query is over.
-template <bool ANY>
+// SORT: nearest child first. Closest hits need it to end early, and any-hit
+// queries meet their blocker sooner (1.5M rays into 1,000 instances 1.38 -> 1.23
+// ms, the cloud's shadow rays 4.44 -> 3.56); transmittance queries visit
+// everything on the segment whatever the order and go without (forest shadow
+// rays 23.2 with, 20.5 ms).
+template <bool SORT>
 __device__ __forceinline__ bool op_node(const DevScene& S, PhaseState& ps, TravStack& st, uint32_t* err) {
     TravState& ts = ps.ts;
     NodeHits h;
@@ -518,7 +523,7 @@ __device__ __forceinline__ bool op_node(const DevScene& S, PhaseState& ps, TravS
         atomicOr(err, RT_DEVERR_STACK);
         return true;
     }
-    if (ANY) {
+    if (!SORT) {
         const int k0 = __ffs(m) - 1;
         int at = st.sp;
 #pragma unroll
