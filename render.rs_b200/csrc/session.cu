@@ -829,7 +829,8 @@ int rt_denoise(rt_session* s, float* rgb) {
         rc = fail(RT_ERR_CUDA, "denoise read-back failed");
     pool_free(d, s->stream);
     if (o) pool_free(o, s->stream);
-    cudaStreamSynchronize(s->stream);
+    const cudaError_t done = cudaStreamSynchronize(s->stream);
+    if (!rc && done != cudaSuccess) rc = fail(RT_ERR_CUDA, std::string("denoise: ") + cudaGetErrorString(done));
     return rc;
 }
 
