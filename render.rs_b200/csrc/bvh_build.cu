@@ -141,40 +141,65 @@ __device__ __forceinline__ double split_boundary(double amin, double aext, int b
 }
 
 // SAH over 16 bins (7 words each: lo keys, hi keys, count), the host
-// builder's sweep: (cost, bin after which to split).
+// builder's sweep: (cost, bin after which to split), the same on every lane.
+// Called by a whole warp, a lane per bin: the boxes and counts left and right of
+// each split are prefix and suffix scans (keys order as their floats do), each
+// lane prices its split, and the cheapest, the first among equals, wins. A sweep
+// by every lane for itself was most of a small node's time (k_subtrees of a
+// 300,000-triangle mesh 842 us).
 __device__ double sah_sweep(const uint32_t* bins, uint32_t count, int* best_bin_out) {
-    float rlo[BINS][3], rhi[BINS][3];
-    float alo[3] = {INFINITY, INFINITY, INFINITY}, ahi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int i = BINS - 1; i >= 1; i--) {
+    const int i = (int)(threadIdx.x & 31u);
+    uint32_t left[7], right[7];
+#pragma unroll
+    for (int w = 0; w < 7; w++) {
+        const uint32_t none = w < 3 ? KEY_F_POS_INF : w < 6 ? KEY_F_NEG_INF : 0u;
+        left[w] = right[w] = i < BINS ? bins[i * 7 + w] : none;
+    }
+    auto join = [](uint32_t* x, const uint32_t* y) {
+#pragma unroll
+        for (int w = 0; w < 7; w++) x[w] = w < 3 ? min(x[w], y[w]) : w < 6 ? max(x[w], y[w]) : x[w] + y[w];
+    };
+#pragma unroll
+    for (int off = 1; off < BINS; off <<= 1) {
+        uint32_t up[7], down[7];
+#pragma unroll
+        for (int w = 0; w < 7; w++) {
+            up[w] = __shfl_up_sync(0xFFFFFFFFu, left[w], off);
+            down[w] = __shfl_down_sync(0xFFFFFFFFu, right[w], off);
+        }
+        if (i >= off) join(left, up);
+        if (i + off < 32) join(right, down);
+    }
+    // Right of the split after bin i: the suffix from bin i + 1.
+#pragma unroll
+    for (int w = 0; w < 7; w++) right[w] = __shfl_down_sync(0xFFFFFFFFu, right[w], 1);
+    double cost = INFINITY;
+    const uint32_t lc = left[6], rc = count - lc;
+    if (i < BINS - 1 && lc != 0 && rc != 0) {
+        float llo[3], lhi[3], rlo[3], rhi[3];
+#pragma unroll
         for (int a = 0; a < 3; a++) {
-            float l = fval(bins[i * 7 + a]), h = fval(bins[i * 7 + 3 + a]);
-            alo[a] = l < alo[a] ? l : alo[a];
-            ahi[a] = h > ahi[a] ? h : ahi[a];
-            rlo[i][a] = alo[a];
-            rhi[i][a] = ahi[a];
+            llo[a] = fval(left[a]);
+            lhi[a] = fval(left[3 + a]);
+            rlo[a] = fval(right[a]);
+            rhi[a] = fval(right[3 + a]);
+        }
+        const double c = __dadd_rn(__dmul_rn(area_d(llo, lhi), (double)lc), __dmul_rn(area_d(rlo, rhi), (double)rc));
+        if (c < cost) cost = c;
+    }
+    int bin = cost < INFINITY ? i : 0;
+#pragma unroll
+    for (int off = 1; off < BINS; off <<= 1) {
+        const double c = __shfl_xor_sync(0xFFFFFFFFu, cost, off);
+        const int k = __shfl_xor_sync(0xFFFFFFFFu, bin, off);
+        if (c < cost || (c == cost && k < bin)) {
+            cost = c;
+            bin = k;
         }
     }
-    double best = INFINITY;
-    int best_bin = 0;
-    float llo[3] = {INFINITY, INFINITY, INFINITY}, lhi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    uint32_t lc = 0;
-    for (int i = 0; i < BINS - 1; i++) {
-        for (int a = 0; a < 3; a++) {
-            float l = fval(bins[i * 7 + a]), h = fval(bins[i * 7 + 3 + a]);
-            llo[a] = l < llo[a] ? l : llo[a];
-            lhi[a] = h > lhi[a] ? h : lhi[a];
-        }
-        lc += bins[i * 7 + 6];
-        uint32_t rc = count - lc;
-        if (lc == 0 || rc == 0) continue;
-        double cost = __dadd_rn(__dmul_rn(area_d(llo, lhi), (double)lc), __dmul_rn(area_d(rlo[i + 1], rhi[i + 1]), (double)rc));
-        if (cost < best) {
-            best = cost;
-            best_bin = i;
-        }
-    }
-    *best_bin_out = best_bin;
-    return best;
+    cost = __shfl_sync(0xFFFFFFFFu, cost, 0);
+    *best_bin_out = __shfl_sync(0xFFFFFFFFu, bin, 0);
+    return cost;
 }
 
 __device__ __forceinline__ void init_bins(uint32_t* bins, uint32_t k) {
@@ -410,10 +435,10 @@ __global__ void __launch_bounds__(LB) k_bin(LevelArgs A) {
     }
 }
 
-// Split decision per job (the host builder's split_node rules).
+// Split decision per job (the host builder's split_node rules), a warp each.
 __global__ void k_decide(LevelArgs A, uint32_t n_jobs, uint32_t max_leaf) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n_jobs) return;
+    const uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (j >= n_jobs) return;  // the whole warp leaves together
     const Job J = A.jobs[j];
     JobInfo I = A.info[j];
     I.m = 0;
@@ -441,7 +466,7 @@ __global__ void k_decide(LevelArgs A, uint32_t n_jobs, uint32_t max_leaf) {
             }
         }
     }
-    A.info[j] = I;
+    if ((threadIdx.x & 31u) == 0) A.info[j] = I;
 }
 
 __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* sh) {
@@ -1232,7 +1257,7 @@ int build_binary_device(Scratch& D, BPrim* P0, BPrim* P1, uint32_t n,
         LevelArgs A{jobs[cur], info[cur], chunk_job, chunk_left, acc_box[cur], acc_cb[cur], acc_bin[cur], {P0, P1}};
         k_bounds<<<nch, LB, 0, st>>>(A);
         k_bin<<<nch, LB, 0, st>>>(A);
-        k_decide<<<blocks_for(J, JB), JB, 0, st>>>(A, J, max_leaf);
+        k_decide<<<blocks_for(32ull * J, JB), JB, 0, st>>>(A, J, max_leaf);
         k_count<<<nch, LB, 0, st>>>(A);
         k_scatter<<<nch, LB, 0, st>>>(A);
         BV_TRY(cudaMemsetAsync(&counters[1], 0, 8, st));
