@@ -1615,12 +1615,14 @@ __global__ void __launch_bounds__(BLOCK) k_sss(DevScene S, Paths P, PtConsts C, 
     st.init(stack_sh + threadIdx.x, BLOCK);
     const uint32_t n = P.cnt[CNT_SSS];
     unsigned long long rays = 0;
-    const uint32_t stride = gridDim.x * BLOCK;
-    for (uint32_t j0 = blockIdx.x * BLOCK; j0 < n; j0 += stride) {
-        const uint32_t j = j0 + threadIdx.x;
+    // Few walks are spread over all resident warps (lanes_for).
+    const uint32_t per = lanes_for(n), warp = blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5);
+    const uint32_t stride = gridDim.x * (BLOCK / 32) * per;
+    for (uint32_t j0 = warp * per; j0 < n; j0 += stride) {
+        const uint32_t j = j0 + lane_id();
         uint32_t slot = 0;
         bool extend = false, shadow = false, shadow2 = false;
-        if (j < n) {
+        if (lane_id() < per && j < n) {
             slot = P.q_sss[j];
             const float4 o4 = P.ray_o[slot], d4 = P.ray_d[slot];
             const float4 beta4 = P.beta[slot];
@@ -1804,7 +1806,9 @@ __global__ void __launch_bounds__(BLOCK) k_shadow_walk(DevScene S, Paths P, PtCo
     st.init(stack_sh + threadIdx.x, BLOCK);
     const uint32_t n = P.cnt[CNT_SHADOW];
     unsigned long long rays = 0;
-    for (uint32_t j = blockIdx.x * BLOCK + threadIdx.x; j < n; j += gridDim.x * BLOCK) {
+    // Few paths are spread over all resident warps (lanes_for).
+    const uint32_t per = lanes_for(n), warp = blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5);
+    for (uint32_t j = warp * per + lane_id(); lane_id() < per && j < n; j += gridDim.x * (BLOCK / 32) * per) {
         const uint32_t e = MED ? P.q_sh[j] : (P.q_sh[j] | SH_PRIMARY);
         const uint32_t slot = e & SH_SLOT_MASK;
         const uint4 rs = P.rng[slot];
