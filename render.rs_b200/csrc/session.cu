@@ -575,7 +575,7 @@ int rt_render_samples(rt_session* s, uint32_t sample_start, uint32_t count) {
     // bounce (cutouts skipped in shade waves, volume-hull crossings).
     const bool skip_waves = (s->S.any_presence && !C.pres_in_trav) || s->S.n_media;
     uint32_t waves = C.max_depth + (skip_waves ? RT_MAX_PRESENCE_SKIPS : 0u);
-    const int trav_grid = s->trav_grid, shade_grid = s->sm_count * 8;
+    const int trav_grid = s->trav_grid, shade_grid = s->sm_count * 4, gather_grid = s->sm_count * 8;
     const uint32_t batch = 1u << 16;  // training records per Adam step
     CUDA_TRY(cudaMemsetAsync(s->stats, 0, 32, st));
     float ms_ext = 0, ms_sh = 0, ms_shade = 0;
@@ -635,7 +635,7 @@ int rt_render_samples(rt_session* s, uint32_t sample_start, uint32_t count) {
             if (s->guide) {
                 // Network inputs for this wave's guided vertices, then inference.
                 CUDA_TRY(cudaMemsetAsync(P.g_cnt, 0, 4, st));
-                k_guide_gather<<<shade_grid, 128, 0, st>>>(s->S, P, s->params.guide_depth);
+                k_guide_gather<<<gather_grid, 128, 0, st>>>(s->S, P, s->params.guide_depth);
                 float* raw = nullptr;
                 int grc = guide_infer_counted(s->guide, P.g_rec, P.g_cnt, P.P, &raw, st);
                 if (grc) return fail(grc, rt_guide_last_error());
