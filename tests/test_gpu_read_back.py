@@ -1,0 +1,48 @@
+"""Reading results back: sizes below and above the pinned path's limit, odd ones, and two sessions read from two
+threads at once (one of them finds the pinned slots taken)."""
+import threading
+
+import numpy as np
+import pytest
+
+from rtcuda import PtSession, abi, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(g):
+    acc, img, aux, film = g.sum_and_weight(), g.image(), g.aux(), g.film_array()
+    assert np.array_equal(img, (acc[..., :3] / acc[..., 3:]).astype(np.float32))
+    assert np.array_equal(film[..., 0:3], img)
+    hits = aux[..., 11]
+    assert np.array_equal(film[..., 16], aux[..., 7]) and (hits <= acc[..., 3]).all()
+    assert (acc[..., 3] == acc[0, 0, 3]).all()
+
+
+@pytest.mark.parametrize("w,h", [(64, 48), (591, 592), (1031, 1021), (1920, 1080)])
+def test_layers_agree(w, h):
+    with PtSession(scenes.cornell_box(w, h), abi.make_params(max_depth=2, aovs=True)) as g:
+        g.render_samples(0, 1)
+        _check(g)
+        g.render_samples(1, 2)
+        _check(g)
+
+
+def test_two_threads():
+    errors = []
+
+    def work(k):
+        try:
+            with PtSession(scenes.cornell_box(1300 + k, 900), abi.make_params(max_depth=2, aovs=True)) as g:
+                g.render_samples(k, 1)
+                for _ in range(6):
+                    _check(g)
+        except Exception as e:  # reported by the main thread
+            errors.append(e)
+
+    t = [threading.Thread(target=work, args=(k,)) for k in range(3)]
+    for x in t:
+        x.start()
+    for x in t:
+        x.join()
+    assert not errors, errors
