@@ -216,9 +216,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) k_guide_fwd(GuideDev G, const 
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     uint32_t r[32];
-                    tmem_ld16_nowait(lane_addr + 32 * h, r);
-                    tmem_ld16_nowait(lane_addr + 32 * h + 16, r + 16);
-                    tmem_ld_wait();
+                    tmem_ld32(lane_addr + 32 * h, r);
 #pragma unroll
                     for (int c = 0; c < 4; c++) {
                         const int k = 32 * h + 8 * c;
@@ -235,19 +233,20 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) k_guide_fwd(GuideDev G, const 
                     }
                 }
             } else {
-                uint32_t r[G_OUT];
-#pragma unroll
-                for (int c = 0; c < G_OUT / 16; c++) tmem_ld16_nowait(lane_addr + c * 16, r + 16 * c);
-                tmem_ld_wait();
+                uint32_t r[32];
+                float last[16];
+                tmem_ld32(lane_addr, r);
+                tmem_ld16(lane_addr + 32, last);
                 if (valid) {
                     float v[G_OUT];
 #pragma unroll
                     for (int k = 0; k < G_OUT; k += 4) {
                         const float4 b4 = *reinterpret_cast<const float4*>(&bias[b_off(3) + k]);
-                        v[k] = __uint_as_float(r[k]) + b4.x;
-                        v[k + 1] = __uint_as_float(r[k + 1]) + b4.y;
-                        v[k + 2] = __uint_as_float(r[k + 2]) + b4.z;
-                        v[k + 3] = __uint_as_float(r[k + 3]) + b4.w;
+                        auto raw = [&](int i) { return i < 32 ? __uint_as_float(r[i]) : last[i - 32]; };
+                        v[k] = raw(k) + b4.x;
+                        v[k + 1] = raw(k + 1) + b4.y;
+                        v[k + 2] = raw(k + 2) + b4.z;
+                        v[k + 3] = raw(k + 3) + b4.w;
                     }
                     if (MODE == FWD_RENDER) {
                         mixture_decode_store(v, out + (size_t)row * G_OUT);
