@@ -742,8 +742,9 @@ struct rt_guide {
     }
 };
 
+// `out`: where the outputs go (48 floats a record, 16-byte aligned), g->out when null.
 static int launch_forward(rt_guide* g, const float* rec, uint32_t n, int mode, cudaStream_t st,
-                          BatchSel B = BatchSel{nullptr, 0, 1}) {
+                          BatchSel B = BatchSel{nullptr, 0, 1}, float* out = nullptr) {
     if (n == 0) return 0;
     int rc = g->ensure(n, mode == FWD_TRAIN);
     if (rc) return rc;
@@ -751,12 +752,13 @@ static int launch_forward(rt_guide* g, const float* rec, uint32_t n, int mode, c
     k_guide_encode<<<enc_grid, 256, 0, st>>>(g->G, rec, n, B, g->X0);
     uint32_t tiles = (n + TILE - 1) / TILE;
     int grid = (int)std::min<uint32_t>(tiles, (uint32_t)g->sms);
+    if (!out) out = g->out;
     if (mode == FWD_TRAIN)
-        k_guide_fwd<FWD_TRAIN><<<grid, FWD_THREADS, F_BYTES, st>>>(g->G, g->X0, n, B, g->acts, g->out, g->err);
+        k_guide_fwd<FWD_TRAIN><<<grid, FWD_THREADS, F_BYTES, st>>>(g->G, g->X0, n, B, g->acts, out, g->err);
     else if (mode == FWD_RENDER)
-        k_guide_fwd<FWD_RENDER><<<grid, FWD_THREADS, F_BYTES, st>>>(g->G, g->X0, n, B, g->acts, g->out, g->err);
+        k_guide_fwd<FWD_RENDER><<<grid, FWD_THREADS, F_BYTES, st>>>(g->G, g->X0, n, B, g->acts, out, g->err);
     else
-        k_guide_fwd<FWD_RAW><<<grid, FWD_THREADS, F_BYTES, st>>>(g->G, g->X0, n, B, g->acts, g->out, g->err);
+        k_guide_fwd<FWD_RAW><<<grid, FWD_THREADS, F_BYTES, st>>>(g->G, g->X0, n, B, g->acts, out, g->err);
     G_TRY(cudaGetLastError());
     return 0;
 }
@@ -974,9 +976,10 @@ int rt_guide_info(rt_guide* g, float* res_out, float* lo_out, float* inv_ext_out
 int rt_guide_infer_device(rt_guide* g, const float* rec, uint32_t n, float* raw_out, void* stream) {
     if (!g || (n && (!rec || !raw_out))) return gfail(-1, "NULL argument");
     cudaStream_t st = (cudaStream_t)stream;
-    int rc = launch_forward(g, rec, n, FWD_RAW, st);
+    const bool direct = ((uintptr_t)raw_out & 15u) == 0;  // the kernel stores 16 bytes at a time
+    int rc = launch_forward(g, rec, n, FWD_RAW, st, BatchSel{nullptr, 0, 1}, direct ? raw_out : nullptr);
     if (rc) return rc;
-    if (n) G_TRY(cudaMemcpyAsync(raw_out, g->out, (size_t)n * G_OUT * 4, cudaMemcpyDeviceToDevice, st));
+    if (n && !direct) G_TRY(cudaMemcpyAsync(raw_out, g->out, (size_t)n * G_OUT * 4, cudaMemcpyDeviceToDevice, st));
     return 0;
 }
 

@@ -29,12 +29,14 @@ namespace rt {
 
 enum : uint32_t { CLS_MISS = N_MAT_CLASSES, N_QUEUES = N_MAT_CLASSES + 1 };
 
-// Counter words (uint32) in Paths::cnt.
+// Counter words (uint32) in Paths::cnt. Every wave has a block of its own, all
+// cleared at the start of the slab, and Paths::cnt points at the current one: a
+// wave's extension rays are the CNT_EXT_OUT of the block before it (ray
+// generation fills block 0), so no launch resets or swaps counters between waves.
 enum : uint32_t {
-    CNT_EXT_IN = 0,
-    CNT_EXT_OUT = 1,
-    CNT_SHADOW = 2,
-    CNT_CLASS = 3,                  // N_QUEUES words
+    CNT_EXT_OUT = 0,
+    CNT_SHADOW = 1,
+    CNT_CLASS = 2,                  // N_QUEUES words
     CNT_FETCH_EXT = CNT_CLASS + N_QUEUES,
     CNT_FETCH_SH = CNT_FETCH_EXT + 1,
     CNT_SSS = CNT_FETCH_SH + 1,     // subsurface walks queued this wave
@@ -354,7 +356,7 @@ __global__ void k_raygen(DevScene S, Paths P, PtConsts C) {
     if (adaptive) {
         // Converged pixels get no path; live ones are compacted into the queue.
         const bool live = i < P.P && !pixel_converged(C, pixel, sample);
-        push_queue(P.q_ext[0], &P.cnt[CNT_EXT_IN], i, live);
+        push_queue(P.q_ext[0], &P.cnt[CNT_EXT_OUT], i, live);
         if (i >= P.P) return;
         if (!live) {
             P.L[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -433,7 +435,7 @@ __global__ void k_raygen(DevScene S, Paths P, PtConsts C) {
     }
     if (!adaptive) {
         P.q_ext[0][i] = i;
-        if (i == 0) P.cnt[CNT_EXT_IN] = P.P;
+        if (i == 0) P.cnt[CNT_EXT_OUT] = P.P;
     }
 }
 
@@ -784,7 +786,7 @@ __global__ void __launch_bounds__(BLOCK, RT_TRAV_MIN_BLOCKS) k_extend(DevScene S
     TravStack st;
     st.init(stack_sh + threadIdx.x, BLOCK);
     const uint32_t* q = P.q_ext[qsel];
-    const uint32_t n = P.cnt[CNT_EXT_IN];
+    const uint32_t n = (P.cnt - CNT_WORDS)[CNT_EXT_OUT];  // queued by the wave before
     unsigned long long rays = 0;
     uint32_t slot = 0;
     uint32_t qk = 0xFFFFFFFFu;  // closest quadric of this lane's ray (scene/mod.rs:105-146), ~0 for none
@@ -1608,7 +1610,6 @@ __global__ void __launch_bounds__(BLOCK, TRANS || QUAD || MOT ? RT_TRAV_MIN_BLOC
     if (rays) atomicAdd(&P.stats[1], rays);
 }
 
-// Between waves: the next extend queue becomes the current one.
 // ---- subsurface walks ------------------------------------------------------------------
 // One thread per walk queued by k_shade (pt/mod.rs:794-892): isotropic
 // scattering through the material's homogeneous Burley-fit medium, one
@@ -1845,20 +1846,6 @@ __global__ void __launch_bounds__(BLOCK) k_shadow_walk(DevScene S, Paths P, PtCo
         }
     }
     if (rays) atomicAdd(&P.stats[1], rays);
-}
-
-__global__ void k_wave_prep(uint32_t* cnt) {
-    uint32_t t = threadIdx.x;
-    if (t == 0) {
-        cnt[CNT_EXT_IN] = cnt[CNT_EXT_OUT];
-        cnt[CNT_EXT_OUT] = 0;
-        cnt[CNT_SHADOW] = 0;
-        cnt[CNT_FETCH_EXT] = 0;
-        cnt[CNT_FETCH_SH] = 0;
-        cnt[CNT_SSS] = 0;
-        cnt[CNT_FETCH_SHADE] = 0;
-    }
-    if (t < N_QUEUES) cnt[CNT_CLASS + t] = 0;
 }
 
 // ---- accumulate ------------------------------------------------------------------------

@@ -179,6 +179,9 @@ cudaError_t read_back(void* dst, const void* src, size_t bytes, int device, cuda
     return (cudaError_t)error.load();
 }
 
+// Waves of a slab at most: a bounce each, and the surfaces passed without one.
+constexpr uint32_t RT_MAX_WAVES = 255u + RT_MAX_PRESENCE_SKIPS;
+
 #ifndef RT_TRAV_BLOCK
 #define RT_TRAV_BLOCK 128
 #endif
@@ -217,6 +220,7 @@ struct rt_session {
     uint64_t device_bytes = 0;
     // path state
     Paths paths{};
+    uint32_t* counters = nullptr;  // CNT_WORDS per wave of a slab, and before the first
     uint32_t slab_samples = 1;     // sample passes per slab
     double* lum_stats = nullptr;   // per pixel: luminance sum, sum of squares, count, pad
     float adaptive_tol = 0.0f;     // rt_set_adaptive
@@ -495,7 +499,7 @@ int rt_session_create(const rt_scene_desc* scene, const rt_params* params, rt_se
     rc = rc ? rc : s->alloc(&Pp.q_ext[1], P);
     rc = rc ? rc : s->alloc(&Pp.q_cls, P * N_QUEUES);
     rc = rc ? rc : s->alloc(&Pp.q_sh, P);
-    rc = rc ? rc : s->alloc(&Pp.cnt, CNT_WORDS);
+    rc = rc ? rc : s->alloc(&s->counters, CNT_WORDS * (1 + RT_MAX_WAVES));
     rc = rc ? rc : s->alloc(&s->stats, 4);
     rc = rc ? rc : s->alloc(&s->err, 1);
     rc = rc ? rc : s->alloc(&s->fetch, 1);
@@ -688,11 +692,13 @@ int rt_render_samples(rt_session* s, uint32_t sample_start, uint32_t count) {
         if (train) k = (uint32_t)std::min<uint64_t>(k, guide_train_budget(s->params.guide_train_passes) - s->guide_trained_passes);
         C.train = train ? 1u : 0u;
         if (train) P.tr_tag++;  // new tag: the training records of this slab
-        CUDA_TRY(cudaMemsetAsync(P.cnt, 0, CNT_WORDS * 4, st));
+        P.cnt = s->counters;
+        CUDA_TRY(cudaMemsetAsync(P.cnt, 0, CNT_WORDS * 4 * (1 + (size_t)waves), st));
         k_raygen<<<(slab_paths + 255) / 256, 256, 0, st>>>(s->S, P, C);
         launches++;
         for (uint32_t w = 0; w < waves; w++) {
             uint32_t qin = w & 1u, qout = qin ^ 1u;
+            P.cnt = s->counters + CNT_WORDS * (1 + w);
             CUDA_TRY(cudaEventRecord(s->evpool[ei], st));
             const bool quad = extra_geometry(s), mot = s->S.motion != 0;
             if (C.pres_in_trav && mot) k_extend<TRAV_BLOCK, true, true, true><<<trav_grid, TRAV_BLOCK, 0, st>>>(s->S, P, qin);
@@ -737,8 +743,7 @@ int rt_render_samples(rt_session* s, uint32_t sample_start, uint32_t count) {
             else
                 launch_shadow<false>(s, P, C, st);
             CUDA_TRY(cudaEventRecord(s->evpool[ei + 3], st));
-            k_wave_prep<<<1, 32, 0, st>>>(P.cnt);
-            launches += 4;
+            launches += 3;
             ei += 4;
         }
         k_accumulate<<<(s->npix + 255) / 256, 256, 0, st>>>(P, C, k, s->accum, s->aux);
