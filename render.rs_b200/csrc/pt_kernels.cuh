@@ -130,8 +130,10 @@ struct PtConsts {
 #define RT_RAY_OFFSET 1e-4f
 // Resident 128-thread blocks per SM the traversal kernels ask for. They are
 // bound by latency and issue at a few warps per scheduler, so blocks count as
-// long as nothing spills: closest-hit and any-hit kernels without cutouts,
-// quadrics or motion fit 80 registers (six blocks), the others 96 (five).
+// long as little spills: closest-hit and any-hit kernels without cutouts,
+// quadrics or motion fit 80 registers (six blocks; 4.19M closest-hit rays 5.66 ->
+// 5.36 ms, 1.5M any-hit rays 1.51 -> 1.38), the others 96 (five). k_extend
+// chooses by the size of the scene.
 #define RT_TRAV_MIN_BLOCKS 5
 #define RT_TRAV_PLAIN_BLOCKS 6
 #define RT_MAX_PRESENCE_SKIPS 16u
@@ -779,20 +781,27 @@ __device__ __forceinline__ void ray_pump(const DevScene& S, uint32_t n, uint32_t
 // (leaf_coop, PRES) instead of by the shade kernel's skip waves.
 // QUAD: the scene has quadrics or curve sets; MOT: motion blur (rays carry
 // their path's shutter time; launched with QUAD).
-template <int BLOCK, bool PRES, bool QUAD = false, bool MOT = false>
-__global__ void __launch_bounds__(BLOCK, RT_TRAV_MIN_BLOCKS) k_extend(DevScene S, Paths P, uint32_t qsel) {
+// BLOCKS: resident blocks per SM. Six leave 80 registers (28 bytes spill), which
+// pays where rays wait for nodes from L2: with RT_EXTEND_LARGE nodes and more the
+// closest hits of the cloud's frame take 11.0 ms instead of 11.4 and of the
+// instanced scene's 15.2 instead of 15.8. Scenes of a few nodes find them in L1
+// and lose with six (Cornell 0.90 -> 0.94 ms), so they keep five.
+#define RT_EXTEND_LARGE 4096u
+template <int BLOCK, bool PRES, bool QUAD = false, bool MOT = false, int BLOCKS = RT_TRAV_MIN_BLOCKS>
+__global__ void __launch_bounds__(BLOCK, BLOCKS) k_extend(DevScene S, Paths P, uint32_t qsel) {
     __shared__ uint2 stack_sh[RT_SH_STACK * BLOCK];
     __shared__ LeafShared leaf_sh[BLOCK / 32];
     TravStack st;
     st.init(stack_sh + threadIdx.x, BLOCK);
     const uint32_t* q = P.q_ext[qsel];
     const uint32_t n = (P.cnt - CNT_WORDS)[CNT_EXT_OUT];  // queued by the wave before
-    unsigned long long rays = 0;
-    uint32_t slot = 0;
+    constexpr bool RELOAD = BLOCKS > RT_TRAV_MIN_BLOCKS;  // the slot is read again at the end, not kept
+    uint32_t rays = 0, slot_kept = 0;
     uint32_t qk = 0xFFFFFFFFu;  // closest quadric of this lane's ray (scene/mod.rs:105-146), ~0 for none
     float qt = 0.0f;            // its parametric distance
     auto load = [&](uint32_t j, float3& o, float3& d, float& tmax, uint64_t& seed, float& time) {
-        slot = q[j];
+        const uint32_t slot = q[j];
+        slot_kept = slot;
         float4 o4 = P.ray_o[slot], d4 = P.ray_d[slot];
         o = xyz(o4);
         d = xyz(d4);
@@ -815,8 +824,9 @@ __global__ void __launch_bounds__(BLOCK, RT_TRAV_MIN_BLOCKS) k_extend(DevScene S
             if (qk != 0xFFFFFFFFu) tmax = qt = tw / dl;
         }
     };
-    auto finish = [&](bool done, uint32_t, const TravState& ts) {
+    auto finish = [&](bool done, uint32_t j, const TravState& ts) {
         uint32_t cls = CLS_MISS;
+        const uint32_t slot = !RELOAD ? slot_kept : done ? q[j] : 0u;
         if (done) {
             const TraceHit& h = ts.hit;
             uint32_t uv = (uint32_t)__half_as_ushort(__float2half_rn(h.b1)) |
@@ -838,7 +848,7 @@ __global__ void __launch_bounds__(BLOCK, RT_TRAV_MIN_BLOCKS) k_extend(DevScene S
     };
     ray_pump<false, false, PRES, QUAD, MOT>(S, n, &P.cnt[CNT_FETCH_EXT], P.err, st, leaf_sh[threadIdx.x >> 5], load,
                                             finish);
-    if (rays) atomicAdd(&P.stats[0], rays);
+    if (rays) atomicAdd(&P.stats[0], (unsigned long long)rays);
 }
 
 // ---- shade ------------------------------------------------------------------------------

@@ -650,6 +650,7 @@ int rt_render_samples(rt_session* s, uint32_t sample_start, uint32_t count) {
     const bool skip_waves = (s->S.any_presence && !C.pres_in_trav) || s->S.n_media;
     uint32_t waves = C.max_depth + (skip_waves ? RT_MAX_PRESENCE_SKIPS : 0u);
     const int trav_grid = s->trav_grid, shade_grid = s->sm_count * 4, gather_grid = s->sm_count * 8;
+    const bool large = s->host.blas_nodes + s->host.tlas_nodes >= RT_EXTEND_LARGE;
     const uint32_t batch = 1u << 16;  // training records per Adam step
     CUDA_TRY(cudaMemsetAsync(s->stats, 0, 32, st));
     float ms_ext = 0, ms_sh = 0, ms_shade = 0;
@@ -706,6 +707,9 @@ int rt_render_samples(rt_session* s, uint32_t sample_start, uint32_t count) {
             else if (C.pres_in_trav && quad) k_extend<TRAV_BLOCK, true, true><<<trav_grid, TRAV_BLOCK, 0, st>>>(s->S, P, qin);
             else if (C.pres_in_trav) k_extend<TRAV_BLOCK, true><<<trav_grid, TRAV_BLOCK, 0, st>>>(s->S, P, qin);
             else if (quad) k_extend<TRAV_BLOCK, false, true><<<trav_grid, TRAV_BLOCK, 0, st>>>(s->S, P, qin);
+            else if (large)
+                k_extend<TRAV_BLOCK, false, false, false, RT_TRAV_PLAIN_BLOCKS>
+                    <<<s->plain_grid, TRAV_BLOCK, 0, st>>>(s->S, P, qin);
             else k_extend<TRAV_BLOCK, false><<<trav_grid, TRAV_BLOCK, 0, st>>>(s->S, P, qin);
             CUDA_TRY(cudaEventRecord(s->evpool[ei + 1], st));
             if (s->guide) {
