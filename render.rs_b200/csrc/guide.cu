@@ -10,8 +10,9 @@
 //                     the 48 raw outputs, or the decoded mixture when rendering
 //   k_guide_bwd       vMF-mixture loss gradient in registers, then per layer
 //                     two tcgen05 GEMMs: dW = dZ^T H (batch is the K dimension)
-//                     and dH = dZ W; each CTA sums dW/db of its tiles into its
-//                     own f32 row, k_guide_grad_reduce adds the rows in order
+//                     and dH = dZ W; each tile pipeline sums dW/db of its tiles
+//                     into its own f32 row, k_guide_grad_reduce adds the rows in
+//                     a fixed order
 //   k_guide_hash_bwd  scatter-add of d loss / d features into the table
 //                     gradient, in 2^-24 fixed point (integer sums do not
 //                     depend on the order the atomics land in)
