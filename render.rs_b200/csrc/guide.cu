@@ -10,9 +10,8 @@
 //                     the 48 raw outputs, or the decoded mixture when rendering
 //   k_guide_bwd       vMF-mixture loss gradient in registers, then per layer
 //                     two tcgen05 GEMMs: dW = dZ^T H (batch is the K dimension)
-//                     and dH = dZ W; each tile pipeline sums dW/db of its tiles
-//                     into its own f32 row, k_guide_grad_reduce adds the rows in
-//                     a fixed order
+//                     and dH = dZ W; each tile's dW/db go to an f32 row of their
+//                     own, k_guide_grad_reduce adds the rows in a fixed order
 //   k_guide_hash_bwd  scatter-add of d loss / d features into the table
 //                     gradient, in 2^-24 fixed point (integer sums do not
 //                     depend on the order the atomics land in)
@@ -275,48 +274,60 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) k_guide_fwd(GuideDev G, const 
 }
 
 // ---- backward -----------------------------------------------------------------
-// One persistent CTA per SM runs BWD_GROUPS tile pipelines (one warpgroup each)
-// over weights they share, as the forward does. Per layer a pipeline stores dZ
-// and the layer's input H once, row by row in the core-matrix layout, and
-// issues both GEMMs on them: dH = dZ W reads dZ K-major, dW = dZ^T H reads dZ
-// and H transposed (MN-major descriptors over the same bytes), so nothing is
-// copied transposed. With M = 128 the dW GEMM also reads the 64 columns past
-// dZ's last neuron (bytes of the next rows, at the end of the H buffer):
-// accumulator rows nobody reads. The bias gradients are column sums of dZ.
-// A pipeline adds its tiles' dW / db into its own partial row, which is laid out
-// [input][neuron] so the neurons of a warp's lanes are neighbours;
-// k_guide_grad_reduce adds the rows in a fixed order.
+// One CTA per SM runs BWD_GROUPS tile pipelines (one warpgroup and one tile
+// each) over weights they share. Per layer a pipeline stores dZ and the layer's
+// input H once, row by row in the core-matrix layout, H with a column of ones
+// after its last input, and issues both GEMMs on them: dH = dZ W reads dZ
+// K-major, [dW | db]^T = [H | 1]^T dZ reads H and dZ transposed (MN-major
+// descriptors over the same bytes), so nothing is copied transposed and the
+// bias gradients fall out as one more row. With M = 128 that GEMM also reads
+// columns past the ones (bytes of the next rows, or past the end of the
+// buffer): accumulator rows nobody reads. A lane of the accumulator holds an
+// input, so a warp's stores to the row-major partial row are neighbours.
+// Every tile's sums go to a row of their own. The sum over tiles keeps one
+// fixed order whatever the launch shape (k_guide_grad_reduce), so a network
+// trained on the same records stays the same bit for bit.
 // The pass is latency-bound (a chain of four GEMM pairs per tile, nothing near a
 // peak): transposed copies of dZ and H written two bytes at a time, row-strided
-// global sums and two one-tile CTAs per SM took 186 us for 65,536 records; this
-// takes 43.
-// Shared memory: W0 6144 | W1 8192 | W2 8192 | W3 6144 | per group DZ 16384, H 16384.
-// TMEM per group: dW in columns [0, 64), dH in [64, 128).
+// global sums and two one-tile CTAs per SM took 186 us for 65,536 records; with
+// the bias gradients summed from shared memory by threads 43 us, this takes 34.
+// Shared memory: W0 6144 | W1 8192 | W2 8192 | W3 6144 | per group DZ 16384,
+// H [128][72] 18432 | 1024 that the last group's GEMM may read.
+// TMEM per group: [dW | db]^T in columns [0, 64), dH in [64, 128).
 constexpr int BWD_GROUPS = 4, BWD_THREADS = BWD_GROUPS * TILE;
 constexpr uint32_t BWD_TMEM_COLS = 128 * BWD_GROUPS;
-constexpr int B_ACT = F_ACT, B_BYTES = B_ACT + BWD_GROUPS * 32768;
+constexpr uint32_t B_HCOLS = 72, B_GROUP = 16384 + TILE * B_HCOLS * 2;
+constexpr int B_ACT = F_ACT, B_BYTES = B_ACT + BWD_GROUPS * B_GROUP + 1024;
 static_assert(BWD_TMEM_COLS == 512, "backward: TMEM allocation is a power of two");
+// The GEMM over H reads 16 blocks of 8 columns for each 8 rows.
+static_assert((TILE / 8 - 1) * B_HCOLS * 16 + 16 * 128 <= TILE * B_HCOLS * 2 + 1024, "backward: reads past H stay inside");
 
+// Tiles [tile0, tile0 + BWD_GROUPS * gridDim.x), one per pipeline; pipeline p
+// writes partial row p. Rows below `half` go on summing what an earlier launch
+// of the same batch left there (fresh: the first launch).
 __global__ void __launch_bounds__(BWD_THREADS, 1) k_guide_bwd(GuideDev G, const __nv_bfloat16* __restrict__ X0,
                                                               const __nv_bfloat16* __restrict__ acts,
                                                               const float* __restrict__ out,
                                                               const float* __restrict__ rec, uint32_t n, BatchSel B,
-                                                              float* part, float* dX0, float* loss_sum, uint32_t* err) {
+                                                              uint32_t tile0, uint32_t half, float* part, float* dX0,
+                                                              float* loss_sum, uint32_t* err) {
     uint32_t begin;
     n = batch_slice(B, n, begin);
-    if ((uint64_t)blockIdx.x * TILE >= n) return;  // no tile for this CTA
+    if ((uint64_t)(tile0 + blockIdx.x) * TILE >= n) return;  // no tile for this CTA
     rec += 16 * (size_t)begin;
     extern __shared__ __align__(1024) uint8_t sm[];
     __shared__ uint64_t mbar[BWD_GROUPS];
     __shared__ uint32_t tmem_base;
     __shared__ uint32_t group_failed[BWD_GROUPS];
     __shared__ float red[BWD_THREADS / 32];
-    __shared__ float db_half[BWD_GROUPS][64];
     const int tid = threadIdx.x, warp = tid >> 5, grp = tid / TILE, gt = tid % TILE;
     stage_matrix(sm + F_W0, G.w + w_off(0), G_HID, G_IN);
     stage_matrix(sm + F_W1, G.w + w_off(1), G_HID, G_HID);
     stage_matrix(sm + F_W2, G.w + w_off(2), G_HID, G_HID);
     stage_matrix(sm + F_W3, G.w + w_off(3), G_OUT, G_HID);
+    const uint32_t dz_off = B_ACT + B_GROUP * grp, h_off = dz_off + 16384u;
+    const uint4 ones = make_uint4(0x3F80u, 0u, 0u, 0u);  // bf16 1, then zeros
+    *reinterpret_cast<uint4*>(sm + h_off + core_offset(gt, G_HID, B_HCOLS)) = ones;
     if (warp == 0) tmem_alloc(&tmem_base, BWD_TMEM_COLS);
     if (tid < BWD_GROUPS) {
         mbar_init(&mbar[tid], 1);
@@ -328,13 +339,13 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_guide_bwd(GuideDev G, const 
     const uint32_t acc = tmem_base + 128u * grp;
     const uint32_t lane_addr = acc + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t s0 = smem_u32(sm);
-    const uint32_t dz_off = B_ACT + 32768u * grp, h_off = dz_off + 16384u;
-    float* gW = part + (size_t)(grp * gridDim.x + blockIdx.x) * G_NPARAMS;
+    const uint32_t pipe = grp * gridDim.x + blockIdx.x, tile = tile0 + pipe;
+    float* gW = part + (size_t)pipe * G_NPARAMS;
     float* gb = gW + G_NWEIGHTS;
+    const bool fresh = tile0 == 0 || pipe >= half;
     uint32_t phase = 0;
-    bool failed = false, first = true;
     float loss = 0.f;
-    for (uint32_t tile = grp * gridDim.x + blockIdx.x; tile * TILE < n; tile += gridDim.x * BWD_GROUPS) {
+    if ((uint64_t)tile * TILE < n) {
         const uint32_t row = tile * TILE + gt;
         const bool valid = row < n;
         float dz[64];
@@ -358,9 +369,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_guide_bwd(GuideDev G, const 
 #pragma unroll
         for (int l = 3; l >= 0; l--) {
             const int K_in = l_in(l), N_out = l_out(l);
-            // dZ and the layer input H, rows of this tile. H keeps 64 columns a
-            // row in every layer: with another stride in layer 0 a thread's row
-            // would land on rows whose ReLU masks others still read.
+            // dZ and the layer input H, rows of this tile. H keeps its row
+            // length in every layer: with another stride in layer 0 a thread's
+            // row would land on rows whose ReLU masks others still read.
 #pragma unroll
             for (int c = 0; c < 8; c++)
                 if (8 * c < N_out)
@@ -372,8 +383,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_guide_bwd(GuideDev G, const 
 #pragma unroll
             for (int c = 0; c < 8; c++)
                 if (8 * c < K_in)
-                    *reinterpret_cast<uint4*>(sm + h_off + core_offset(gt, 8 * c, G_HID)) =
+                    *reinterpret_cast<uint4*>(sm + h_off + core_offset(gt, 8 * c, B_HCOLS)) =
                         valid ? hp[c] : make_uint4(0, 0, 0, 0);
+            if (l == 0) *reinterpret_cast<uint4*>(sm + h_off + core_offset(gt, G_IN, B_HCOLS)) = ones;
             fence_proxy_async_smem();
             group_sync(grp);
             if (gt == 0) {
@@ -381,52 +393,34 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_guide_bwd(GuideDev G, const 
                 const uint32_t w = s0 + (l == 0 ? F_W0 : l == 1 ? F_W1 : l == 2 ? F_W2 : F_W3);
                 // dH[m][k] = sum_n dZ[m][n] W[n][k]  (N = K_in, K = N_out)
                 tc_gemm_issue_ops(acc + 64u, umma_k_major(s0 + dz_off, N_out), umma_transposed(w, K_in), K_in, N_out);
-                // dW[n][k] = sum_m dZ[m][n] H[m][k]  (M = neurons, N = K_in, K = batch)
-                tc_gemm_issue_ops(acc, umma_transposed(s0 + dz_off, N_out), umma_transposed(s0 + h_off, G_HID), K_in,
-                                  TILE);
+                // dW[n][k] = sum_m dZ[m][n] H[m][k], row k of the accumulator; row K_in: db
+                tc_gemm_issue_ops(acc, umma_transposed(s0 + h_off, B_HCOLS), umma_transposed(s0 + dz_off, N_out),
+                                  N_out, TILE);
                 tc_commit(&mbar[grp]);
             }
-            // db: thread pairs sum a neuron's column, 64 rows each, while the MMAs run.
-            float db = 0.f;
-            const int nn = gt & 63, m0 = (gt >> 6) * 64;
-            if (nn < N_out)
-#pragma unroll 8
-                for (int m = 0; m < 64; m++)
-                    db += __bfloat162float(
-                        *reinterpret_cast<const __nv_bfloat16*>(sm + dz_off + core_offset(m0 + m, nn, N_out)));
-            if (m0) db_half[grp][nn] = db;
             if (!mbar_wait_or_drain(&mbar[grp], phase, G.wait_polls)) group_failed[grp] = 1;
             phase ^= 1u;
             group_sync(grp);
-            if (group_failed[grp]) {
-                failed = true;
-                break;
-            }
+            if (group_failed[grp]) break;
             tc_fence_after();
-            if (gt < 64) {
-                // dW: lane = neuron; column k of the accumulator is input k
-                // (the last 16 of 64 are stale in layer 0, which has 48).
-                float* g = gW + w_off(l) + gt;
+            if (gt < (l > 0 ? 96 : 64)) {  // whole warps: the inputs' lanes and the one after them, with the biases
+                float* at = gt < K_in ? gW + w_off(l) + gt : gb + b_off(l);
+                const int step = gt < K_in ? K_in : 1;
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     uint32_t r[32];
                     tmem_ld32(lane_addr + 32 * h, r);
-                    if (gt < N_out) {
+                    if (gt <= K_in) {
 #pragma unroll
                         for (int k = 0; k < 32; k++)
-                            if (32 * h + k < K_in) {
+                            if (32 * h + k < N_out) {
                                 const float v = __uint_as_float(r[k]);
-                                float* at = g + (32 * h + k) * N_out;
-                                *at = first ? v : *at + v;
+                                float* p = at + (32 * h + k) * step;
+                                *p = fresh ? v : *p + v;
                             }
                     }
                     __syncwarp();
                 }
-                if (gt < N_out) {
-                    const float b = db + db_half[grp][gt];
-                    gb[b_off(l) + gt] = first ? b : gb[b_off(l) + gt] + b;
-                }
-                __syncwarp();
             }
 #pragma unroll
             for (int h = 0; h < (l > 0 ? 2 : 1); h++) {
@@ -438,7 +432,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_guide_bwd(GuideDev G, const 
 #pragma unroll
                     for (int c = 0; c < 4; c++) {
                         const uint4 q =
-                            *reinterpret_cast<const uint4*>(sm + h_off + core_offset(gt, 32 * h + 8 * c, G_HID));
+                            *reinterpret_cast<const uint4*>(sm + h_off + core_offset(gt, 32 * h + 8 * c, B_HCOLS));
                         const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
                         for (int e = 0; e < 4; e++) {
@@ -458,11 +452,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_guide_bwd(GuideDev G, const 
             __syncwarp();
             tc_fence_before();
         }
-        if (failed) {
-            if (gt == 0) atomicOr(err, GERR_WAIT);
-            break;
-        }
-        first = false;
+        if (gt == 0 && group_failed[grp]) atomicOr(err, GERR_WAIT);
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, off);
@@ -480,35 +470,57 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_guide_bwd(GuideDev G, const 
     }
 }
 
-// Adds the pipelines' partial rows (one per tile, at most max_rows) to the MLP
-// gradient: eight threads a parameter take every eighth row, then their sums
-// are added in order. Rows of a failed backward pass are left out.
-constexpr int GR_PARAMS = 64, GR_SLICES = 8;
-__global__ void __launch_bounds__(GR_PARAMS* GR_SLICES) k_guide_grad_reduce(const float* __restrict__ part, uint32_t n,
-                                                                            BatchSel B, uint32_t max_rows, float* gw,
-                                                                            const uint32_t* __restrict__ err) {
-    __shared__ float sum[GR_SLICES][GR_PARAMS];
+// The gradient's order of summation: row r of `half` (two per SM) adds tiles r,
+// r + half, r + 2 half, ... in turn, then the rows are added in turn, all in
+// f32. A launch of the backward pass leaves tiles tile0 + r and tile0 + half + r
+// in rows r and half + r, so a batch of several launches folds the upper rows
+// into the lower ones between them.
+__global__ void __launch_bounds__(256) k_guide_grad_fold(float* part, uint32_t n, BatchSel B, uint32_t tile0,
+                                                         uint32_t half) {
     uint32_t begin;
     n = batch_slice(B, n, begin);
-    const uint32_t rows = min((n + TILE - 1) / TILE, max_rows);
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x, r = blockIdx.y;
+    if (i >= (uint32_t)G_NPARAMS || (uint64_t)(tile0 + half + r) * TILE >= n) return;
+    part[(size_t)r * G_NPARAMS + i] += part[(size_t)(half + r) * G_NPARAMS + i];
+}
+
+// Adds the rows of the last launch (its first tile: tile0) to the MLP gradient.
+// Sixteen warps a block bring 32 parameters' rows to shared memory, all loads
+// in flight together, and one warp adds them in order. Rows of a failed
+// backward pass are left out.
+constexpr int GR_PARAMS = 32, GR_SLICES = 16, GR_ROWS = 304;
+__global__ void __launch_bounds__(GR_PARAMS* GR_SLICES) k_guide_grad_reduce(const float* __restrict__ part, uint32_t n,
+                                                                            BatchSel B, uint32_t tile0, uint32_t half,
+                                                                            float* gw,
+                                                                            const uint32_t* __restrict__ err) {
+    __shared__ float row[GR_ROWS][GR_PARAMS];
+    uint32_t begin;
+    n = batch_slice(B, n, begin);
+    if (*err) return;
+    const uint32_t tiles = (n + TILE - 1) / TILE, rows = min(tiles, half);
     const uint32_t c = threadIdx.x % GR_PARAMS, sl = threadIdx.x / GR_PARAMS;
     const uint32_t i = blockIdx.x * GR_PARAMS + c;
+    const bool own = i < (uint32_t)G_NPARAMS;
     float s = 0.f;
-    if (i < (uint32_t)G_NPARAMS && *err == 0u)
+    for (uint32_t r0 = 0; r0 < rows; r0 += GR_ROWS) {
+        const uint32_t m = min(rows - r0, (uint32_t)GR_ROWS);
+        float lower[GR_ROWS / GR_SLICES], upper[GR_ROWS / GR_SLICES];
+#pragma unroll
+        for (int k = 0; k < GR_ROWS / GR_SLICES; k++) {
+            const uint32_t r = r0 + k * GR_SLICES + sl;
+            const bool in = own && r < rows, pair = in && tile0 + half + r < tiles;
+            lower[k] = in ? part[(size_t)r * G_NPARAMS + i] : 0.f;
+            upper[k] = pair ? part[(size_t)(half + r) * G_NPARAMS + i] : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < GR_ROWS / GR_SLICES; k++) row[k * GR_SLICES + sl][c] = lower[k] + upper[k];
+        __syncthreads();
+        if (sl == 0 && own)
 #pragma unroll 8
-        for (uint32_t b = sl; b < rows; b += GR_SLICES) s += part[(size_t)b * G_NPARAMS + i];
-    sum[sl][c] = s;
-    __syncthreads();
-    if (sl != 0 || i >= (uint32_t)G_NPARAMS) return;
-    for (int k = 1; k < GR_SLICES; k++) s += sum[k][c];
-    // Weights come as [input][neuron] per layer.
-    uint32_t to = i;
-    if (i < (uint32_t)G_NWEIGHTS) {
-        const int l = i < (uint32_t)w_off(1) ? 0 : i < (uint32_t)w_off(2) ? 1 : i < (uint32_t)w_off(3) ? 2 : 3;
-        const uint32_t j = i - w_off(l), N_out = l_out(l), k = j / N_out, nn = j % N_out;
-        to = w_off(l) + nn * l_in(l) + k;
+            for (uint32_t r = 0; r < m; r++) s += row[r][c];
+        __syncthreads();
     }
-    gw[to] += s;
+    if (sl == 0 && own) gw[i] += s;
 }
 
 // Table gradients are summed as integers in units of 2^-24 (each
@@ -565,6 +577,14 @@ struct AdamArgs {
     const float* c;  // device: c[0] = 1/(1-b1^t), c[1] = 1/(1-b2^t), c[2] = 1 when the step runs
 };
 
+// The moving averages, with their roundings written out: what a compiler makes
+// of a sum of two products differs from kernel to kernel, and training is to
+// give the same bits whatever the kernels around it look like.
+__device__ __forceinline__ void adam_moments(const AdamArgs& A, float g, float& m, float& v) {
+    m = __fmaf_rn(1.f - A.b1, g, __fmul_rn(A.b1, m));
+    v = __fmaf_rn(__fmul_rn(1.f - A.b2, g), g, __fmul_rn(A.b2, v));
+}
+
 // Step counter and bias corrections on the device: a step whose batch slice is
 // empty is skipped (no update, no count).
 __global__ void k_guide_adam_tick(BatchSel B, uint32_t cap, AdamArgs A, uint32_t* step, float* c) {
@@ -586,8 +606,8 @@ __global__ void k_guide_adam_mlp(AdamArgs A, float* p, float* g, float* m, float
     if (i >= n_total || A.c[2] == 0.f) return;
     const float c1 = A.c[0], c2 = A.c[1];
     float gi = g[i];
-    float mi = A.b1 * m[i] + (1.f - A.b1) * gi;
-    float vi = A.b2 * v[i] + (1.f - A.b2) * gi * gi;
+    float mi = m[i], vi = v[i];
+    adam_moments(A, gi, mi, vi);
     m[i] = mi;
     v[i] = vi;
     float pi = p[i] - A.lr * (mi * c1) / (sqrtf(vi * c2) + A.eps);
@@ -618,8 +638,7 @@ __global__ void __launch_bounds__(256) k_guide_adam_table(AdamArgs A, float4* __
     for (int k = 0; k < 4; k++) {
         if (q[k] == 0ull) continue;
         const float gi = from_fix(q[k]);
-        mv[k] = A.b1 * mv[k] + (1.f - A.b1) * gi;
-        vv[k] = A.b2 * vv[k] + (1.f - A.b2) * gi * gi;
+        adam_moments(A, gi, mv[k], vv[k]);
         pv[k] = pv[k] - A.lr * (mv[k] * c1) / (sqrtf(vv[k] * c2) + A.eps);
         h[k] = __half_as_ushort(__float2half_rn(pv[k]));
     }
@@ -681,7 +700,7 @@ struct rt_guide {
     __nv_bfloat16* w16 = nullptr;
     float* t32 = nullptr;      // table master (levels * T * 2)
     unsigned long long* gt = nullptr;  // table gradient, 2^-24 fixed point
-    float* part = nullptr;     // backward pipelines' dW / db partial rows (sms x BWD_GROUPS x G_NPARAMS)
+    float* part = nullptr;     // a launch's tiles' dW / db (sms x BWD_GROUPS rows of G_NPARAMS)
     float* mt = nullptr;
     float* vt = nullptr;
     __half* t16 = nullptr;
@@ -767,12 +786,17 @@ static int launch_forward(rt_guide* g, const float* rec, uint32_t n, int mode, c
 static int launch_backward(rt_guide* g, const float* rec, uint32_t n, cudaStream_t st,
                            BatchSel B = BatchSel{nullptr, 0, 1}) {
     uint32_t tiles = (n + TILE - 1) / TILE;
-    int grid = (int)std::min<uint32_t>(tiles, (uint32_t)g->sms);
+    const uint32_t sms = (uint32_t)g->sms, half = BWD_GROUPS / 2 * sms;
     G_TRY(cudaMemsetAsync(g->loss, 0, 4, st));
-    k_guide_bwd<<<grid, BWD_THREADS, B_BYTES, st>>>(g->G, g->X0, g->acts, g->out, rec, n, B, g->part, g->dX0, g->loss,
-                                                    g->err);
+    uint32_t tile0 = 0;
+    for (;; tile0 += 2 * half) {
+        k_guide_bwd<<<std::min(tiles - tile0, sms), BWD_THREADS, B_BYTES, st>>>(
+            g->G, g->X0, g->acts, g->out, rec, n, B, tile0, half, g->part, g->dX0, g->loss, g->err);
+        if (tiles - tile0 <= 2 * half) break;
+        k_guide_grad_fold<<<dim3((G_NPARAMS + 255) / 256, half), 256, 0, st>>>(g->part, n, B, tile0, half);
+    }
     k_guide_grad_reduce<<<(G_NPARAMS + GR_PARAMS - 1) / GR_PARAMS, GR_PARAMS * GR_SLICES, 0, st>>>(
-        g->part, n, B, (uint32_t)grid * BWD_GROUPS, g->gw, g->err);
+        g->part, n, B, tile0, half, g->gw, g->err);
     k_guide_hash_bwd<<<(n + HB_WARPS - 1) / HB_WARPS, 32 * HB_WARPS, 0, st>>>(g->G, rec, g->dX0, n, B, g->gt);
     G_TRY(cudaGetLastError());
     return 0;

@@ -1,8 +1,11 @@
 """The training step's backward pass over batch sizes that fill one tile, several CTAs, all their tile pipelines and
 more than one tile per pipeline. Gradients are sums over records, so a batch's gradient is the sum of its chunks'
 (chunks of 1,000 use one pipeline per CTA and are checked against the f64 oracle in test_gpu_guide.py)."""
+import zlib
+
 import numpy as np
 import pytest
+import torch
 
 from rtcuda.guide import Guide, LEVELS, TABLE_ENTRIES
 
@@ -52,3 +55,60 @@ def test_training_is_reproducible():
         out.append(g.params())
         g.close()
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("n", [5, 300 * 128 + 77, 592 * 128, 592 * 128 + 1, 1500 * 128 + 5])
+def test_gradient_keeps_its_order_of_summation(n):
+    """Row r of two per SM adds tiles (128 records) r, r + rows, r + 2 rows, ... in turn, then the rows are added in
+    turn, in f32: bit for bit what the tiles' own gradients give in that order, over batches of one launch of the
+    backward pass, its limit and several."""
+    g = Guide((-1, -1, -1), (1, 1, 1), seed=3)
+    rec = _records(n, n)
+    tiles = [g.grads(rec[k:k + 128], table=False)[2] for k in range(0, n, 128)]
+    rows = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    want = np.zeros_like(tiles[0])
+    for r in range(min(rows, len(tiles))):
+        row = tiles[r].copy()
+        for t in range(r + rows, len(tiles), rows):
+            row += tiles[t]
+        want += row
+    got = g.grads(rec, table=False)[2]
+    g.close()
+    assert np.array_equal(got, want)
+
+
+def test_bias_gradient_is_summed_as_a_weight_of_a_constant_input():
+    """A bias is the weight of an input that is always 1: where a unit of the layer below is 1 for every record, its
+    weights' gradients and the biases' are the same sums, bit for bit."""
+    g = Guide((-1, -1, -1), (1, 1, 1), seed=3)
+    mlp, t = g.params()
+    table = np.random.default_rng(9).normal(scale=0.5, size=t.size)
+    shapes = [(64, 48), (64, 64), (64, 64), (48, 64)]
+    w_at = np.cumsum([0] + [a * b for a, b in shapes])
+    for lv in range(3):   # unit 5 of every hidden layer: no weights, bias 1
+        mlp[w_at[lv]:w_at[lv + 1]].reshape(shapes[lv])[5] = 0.0
+        mlp[w_at[4] + 64 * lv + 5] = 1.0
+    g.set_params(mlp=mlp, table16=np.float16(table).view(np.uint16))
+    rec = _records(40_000, 2)
+    rec[:, 3:6] = (1.0, 0.0, 0.0)   # input 32 of the first layer
+    gm = g.grads(rec, table=False)[2]
+    g.close()
+    for lv, unit in enumerate((32, 5, 5, 5)):
+        o = shapes[lv][0]
+        weights = gm[w_at[lv]:w_at[lv + 1]].reshape(shapes[lv])[:, unit]
+        biases = gm[w_at[4] + 64 * lv:w_at[4] + 64 * lv + o]
+        assert np.abs(biases).max() > 0
+        assert np.array_equal(weights, biases), lv
+
+
+def test_training_gives_the_recorded_network():
+    """Four steps on fixed records give the network recorded here: no change of a kernel's shape may move the order of
+    a sum or where a product is rounded."""
+    g = Guide((-1, -1, -1), (1, 1, 1), seed=3)
+    t = np.random.default_rng(9).normal(scale=0.5, size=LEVELS * TABLE_ENTRIES * 2)
+    g.set_params(table16=np.float16(t).view(np.uint16))
+    for k in range(4):
+        g.train_step(_records(60_000, k))
+    mlp, table = g.params()
+    g.close()
+    assert (zlib.crc32(mlp.tobytes()), zlib.crc32(table.tobytes())) == (1770624645, 2885379321)
