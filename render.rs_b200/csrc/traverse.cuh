@@ -316,14 +316,20 @@ struct NodeHits {
 // mantissa of 2^15), which leaves a permute and a fused multiply-add per plane;
 // the near and far bytes are chosen by the direction's sign once per node, so
 // an axis needs no minimum and maximum per child.
-// Rounding: with u = 2^-24, c = (p - o) / d is off by at most 4u|c| (difference,
-// approximate reciprocal, product), C by u (|c| + 32768|A|) more, the product's A
-// by 2u per unit of q|A| <= 255|A|, and the sum by u|t| with |t| <= |c| + 255|A|:
-// in all under 16u|c| + 2^-8|A| per plane. Cn and Cf are moved outward by
-// 2^-20|c| + 2^-7|A|, more than that with their own rounding, so a box the ray
-// meets is never missed and a child box grows by less than a hundredth of the
-// grid step it was already rounded out to. Overflows give infinities or NaN,
-// which fmaxf and fminf drop: the axis then cuts nothing.
+// Rounding, with u = 2^-24 and c = (p - o) / d: c is off by at most 6u|c|
+// (difference, approximate reciprocal, product), C by u (|c| + 32768|A|) more, the
+// product q A by 4u * 255|A|, the sum by u|t| with |t| <= |c| + 255|A|, and moving
+// C outward by another u (|c| + 32768|A|); A's own error cancels in all but its q
+// multiples, and results below the normal range add less than 2^-141: in all under
+// 10u|c| + 2^-7.9|A| + 2^-141. Cn and Cf are moved outward by
+// 2^-20|c| + 2^-7|A| + 2^-134, so a box the ray meets is never missed. A child box
+// grows by 2^-7 grid steps and 2^-20 of its node's distance along the axis (the
+// larger part from 2^13 steps on: fine nodes seen from afar).
+// Where a plane's distance nears 3e38 (wide nodes, direction components near
+// RT_MIN_DIR) A, c or C overflow, C also from finite A and c. The slack holds all
+// three (C too little to matter while finite), so it is infinite then, and Cn and
+// Cf are infinite outward or NaN, which fmaxf and fminf drop: the axis cuts
+// nothing.
 // The kernels are bound by instructions issued: a node step took about 40 per
 // child for exact planes, per-axis minima and a selection loop over the hits,
 // and takes about 20 with the sorting network of op_node. On the 1M-triangle
@@ -339,7 +345,8 @@ __device__ __forceinline__ void test_node(const uint4* __restrict__ nodes, uint3
         const float c = (p - o) * inv;
         A = s * inv;
         const float C = fmaf(-32768.0f, A, c);
-        const float slack = fmaf(fabsf(A), 0x1p-7f, fabsf(c) * 0x1p-20f);
+        const float slack =
+            fmaf(fabsf(C), 0x1p-40f, fmaf(fabsf(A), 0x1p-7f, fmaf(fabsf(c), 0x1p-20f, 0x1p-134f)));
         Cn = C - slack;
         Cf = C + slack;
     };

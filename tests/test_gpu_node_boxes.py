@@ -82,3 +82,35 @@ def test_no_hit_is_lost(centre, scale, far, instanced):
     assert blocked[clear].all()
     # Never behind the closest hit by more than the same rounding along the ray (a nearer edge hit may be taken).
     assert (t[clear] <= want[clear] + 64 * size * 2.0 ** -24).all()
+
+
+@pytest.mark.parametrize("far", [1e15, 5e16, 1e18, 1e22, 1e30])
+def test_a_far_instance_hides_nothing(far):
+    """One instance far away makes the top node's grid step huge: plane distances overflow along the axes on which a
+    ray hardly moves, and no box the ray is in may be lost by that."""
+    pos = scenes.triangle_cloud_mesh(3000, seed=5)[0].astype(np.float32)
+    idx = np.arange(len(pos), dtype=np.uint32).reshape(-1, 3)
+    s = Scene(8, 8)
+    mat = s.add_material(matte((0.5, 0.5, 0.5)))
+    cloud = s.add_mesh(pos, idx)
+    s.add_instance(cloud, mat)
+    for sign in (1.0, -1.0):
+        s.add_instance(cloud, mat, affine(np.eye(3), (sign * far, -sign * far, sign * far)))
+    rng = np.random.default_rng(2)
+    rays = awkward_rays(600, rng, np.zeros(3), 1.0, 2.0)
+    axis = np.zeros((2, 300, 4), np.float32)
+    axis[0, :, :3] = pos.reshape(-1, 3, 3)[rng.integers(0, 3000, 300)].mean(1)
+    axis[1, :, 3] = np.inf
+    for i in range(300):
+        a, sign = i % 3, 1.0 if i % 2 else -1.0
+        axis[0, i, a], axis[1, i, a] = -3.0 * sign, sign
+    rays = np.concatenate([rays, axis], axis=1)
+    with PtSession(s, abi.make_params(max_depth=4, max_paths=64)) as g:
+        prim, inst, t = g.intersect(rays)
+        blocked = g.intersect(rays, any_hit=True)[0]
+    want, edge = brute(pos, rays)
+    clear = np.isfinite(want) & (edge > 16 * 3.5 * 2.0 ** -24 / 0.03 + 1e-5)
+    assert clear[:600].sum() > 60 and clear[600:].sum() > 200
+    assert (prim[clear] != 0xFFFFFFFF).all() and (inst[clear] == 0).all()
+    assert blocked[clear].all()
+    assert (t[clear] <= want[clear] + 64 * 3.5 * 2.0 ** -24).all()
