@@ -17,6 +17,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <float.h>
 #include <stdint.h>
 
 #include "rt_internal.h"
@@ -134,12 +135,14 @@ struct RayPre {
 
 __device__ __forceinline__ float comp(float3 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
 
-// What the box tests need. Direction components below RT_MIN_DIR count as
-// RT_MIN_DIR: a plane distance of 2^-7 grid steps, the least by which test_node
-// widens a slab, then lies at t > 1e15 or so in any scene of visible size. The
-// reciprocals need no more than their widening covers, so the approximate one
+// What the box tests need. A direction component below 1e-25 of the largest counts
+// as that much: over the length of a scene it moves the ray by less than the
+// 2^-7 grid steps of test_node's slack in any node more than 1e-21 of that length
+// wide. The floor is relative, since directions have any length: rays of length
+// 1e-25, or shortened by an instance's transform, are tested along their own
+// direction. It stays a normal number, so that no reciprocal is infinite. The
+// reciprocals need no more than test_node's slack covers, so the approximate one
 // (2 ulp) does; the triangle tests use none of them.
-#define RT_MIN_DIR 1e-20f
 __device__ __forceinline__ float rcp_approx(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -148,7 +151,9 @@ __device__ __forceinline__ float rcp_approx(float x) {
 __device__ __forceinline__ void ray_boxes(RayPre& r, float3 o, float3 d) {
     r.o = o;
     r.d = d;
-    auto safe = [](float x) { return fabsf(x) < RT_MIN_DIR ? copysignf(RT_MIN_DIR, x) : x; };
+    const float largest = fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fabsf(d.z));
+    const float least = fminf(fmaf(largest, 1e-25f, FLT_MIN), 1e14f);  // 1e14: an infinite component
+    auto safe = [&](float x) { return copysignf(fmaxf(fabsf(x), least), x); };
     r.inv = f3(rcp_approx(safe(d.x)), rcp_approx(safe(d.y)), rcp_approx(safe(d.z)));
 }
 // What the triangle tests need; entering an instance computes it, the top level
@@ -325,8 +330,8 @@ struct NodeHits {
 // 2^-20|c| + 2^-7|A| + 2^-134, so a box the ray meets is never missed. A child box
 // grows by 2^-7 grid steps and 2^-20 of its node's distance along the axis (the
 // larger part from 2^13 steps on: fine nodes seen from afar).
-// Where a plane's distance nears 3e38 (wide nodes, direction components near
-// RT_MIN_DIR) A, c or C overflow, C also from finite A and c. The slack holds all
+// Where a plane's distance nears 3e38 (wide nodes, direction components near the
+// floor) A, c or C overflow, C also from finite A and c. The slack holds all
 // three (C too little to matter while finite), so it is infinite then, and Cn and
 // Cf are infinite outward or NaN, which fmaxf and fminf drop: the axis cuts
 // nothing.

@@ -114,3 +114,40 @@ def test_a_far_instance_hides_nothing(far):
     assert (prim[clear] != 0xFFFFFFFF).all() and (inst[clear] == 0).all()
     assert blocked[clear].all()
     assert (t[clear] <= want[clear] + 64 * 3.5 * 2.0 ** -24).all()
+
+
+@pytest.mark.parametrize("length", [1e-28, 1e-25, 1e-21, 1e-12, 1e12, 1e25, 1e30])
+@pytest.mark.parametrize("instanced", [False, True])
+def test_directions_of_any_length(length, instanced):
+    """Directions are used as given: a ray of any length meets what the unit ray meets, at t over its length. Two in
+    three have components a hundred million times below the largest, or none."""
+    pos = scenes.triangle_cloud_mesh(3000, seed=5)[0].astype(np.float32)
+    idx = np.arange(len(pos), dtype=np.uint32).reshape(-1, 3)
+    s = Scene(8, 8)
+    mat = s.add_material(matte((0.5, 0.5, 0.5)))
+    if instanced:
+        s.add_instance(s.add_mesh(pos, idx), mat, affine(np.eye(3) * 3.0, (1.0, 2.0, 3.0)))
+        world = (pos.astype(np.float64) * 3.0 + (1.0, 2.0, 3.0)).astype(np.float32)
+    else:
+        s.add_instance(s.add_mesh(pos, idx), mat)
+        world = pos
+    rng = np.random.default_rng(4)
+    centre, scale = (np.array([1.0, 2.0, 3.0]), 3.0) if instanced else (np.zeros(3), 1.0)
+    rays = awkward_rays(600, rng, centre, scale, 2.0)
+    d = rays[1, :, :3].astype(np.float64)
+    d[np.abs(d) < 1e-8] = 0.0
+    tiny = (d == 0.0) & (rng.uniform(size=d.shape) < 0.5)
+    d = (d + tiny * 1e-9) * length
+    rays[1, :, :3] = d
+    with PtSession(s, abi.make_params(max_depth=4, max_paths=64)) as g:
+        prim, _, t = g.intersect(rays)
+        blocked = g.intersect(rays, any_hit=True)[0]
+    unit = rays.astype(np.float64)
+    unit[1, :, :3] /= length
+    want, edge = brute(world, unit)
+    size = np.abs(centre).max() + 3.0 * scale
+    clear = np.isfinite(want) & (edge > 16 * size * 2.0 ** -24 / (0.03 * scale) + 1e-5)
+    assert clear.sum() > 60
+    assert (prim[clear] != 0xFFFFFFFF).all()
+    assert blocked[clear].all()
+    assert (t[clear].astype(np.float64) * length <= want[clear] + 64 * size * 2.0 ** -24).all()
