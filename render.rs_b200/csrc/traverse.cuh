@@ -8,7 +8,7 @@
 //    (shear to ray space, edge functions, f64 fallback on exact zeros);
 //  * traversal stack: the first 24 entries in shared memory (one column per
 //    thread, bank-conflict free), deeper ones in local memory; a stack deeper
-//    than 128 sets an error bit.
+//    than 512 sets an error bit.
 // The reference's traversal is Bvh::traverse / any_hit (src/accel/bvh.rs:
 // 141-245) over 2-wide nodes with Möller–Trumbore triangles
 // (src/geometry/mesh.rs:117-142) and Instance::intersect (mesh.rs:308-381):
@@ -390,10 +390,16 @@ __device__ __forceinline__ void test_node(const uint4* __restrict__ nodes, uint3
 // time made as many memory requests (10.6M local loads in a 1M-ray batch into the
 // cloud) as the nodes and triangles did: 6.44 -> 5.71 ms for 4.19M closest-hit
 // rays, forest 69 -> 60 ms. 24 or 32 shared entries take the same time.
+// Entries in all: 512. A ray usually needs a few dozen (coincident instances
+// included: seven a level), but a tree can be a comb, whose every level leaves seven
+// children behind: 400 instances, each 1.2 times as far and as large as the one
+// before, take 256 entries with one item per TLAS leaf, where leaves of up to four
+// items took 114 and a limit of 128 was enough. Four times as many cost no time, but
+// a context holds 0.25 GB more local memory.
 #ifndef RT_SH_STACK
 #define RT_SH_STACK 24
 #endif
-#define RT_SPILL (128 - RT_SH_STACK)
+#define RT_SPILL (512 - RT_SH_STACK)
 
 struct TravStack {
     uint2* sh;       // this thread's column: entry k at sh[k * stride]
