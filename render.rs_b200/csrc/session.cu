@@ -119,29 +119,46 @@ struct DeviceScope {
 // is in flight, so the faults and the copies run side by side. One 16 MB buffer,
 // made at the first large read-back and kept for the process; a call that finds
 // it taken copies plainly. A 961 x 541 film (37 MB) came back in 8.1 ms, now 3.6;
-// below 16 MB starting the threads costs more than they save (5.5 MB: 0.4 ms more).
+// below 24 MB starting the threads costs more than they save (5.5 MB: 0.4 ms more,
+// 21 MB into pages in use 1.06 ms against 1.12; 27 MB 1.34 against 1.27).
+// Memory that CUDA knows (pinned, registered, managed) takes the plain copy, which
+// writes it directly: a 1920 x 1080 film (149 MB) into pinned memory 2.8 ms,
+// through the slots 5.5.
 struct ReadBack {
-    static constexpr size_t THREADS = 4, CHUNK = 2u << 20, MIN_BYTES = 16u << 20;
+    static constexpr size_t THREADS = 4, CHUNK = 2u << 20, MIN_BYTES = 24u << 20;
+    // Bytes a thread copies: whole pages, and THREADS of them hold every byte.
+    static constexpr size_t part(size_t bytes) { return ((bytes + THREADS - 1) / THREADS + 4095) & ~(size_t)4095; }
     std::mutex mu;
     char* pinned = nullptr;
 };
+static_assert(ReadBack::THREADS * ReadBack::part(ReadBack::MIN_BYTES + 1) >= ReadBack::MIN_BYTES + 1 &&
+                  ReadBack::THREADS * ReadBack::part(ReadBack::MIN_BYTES + 16383) >= ReadBack::MIN_BYTES + 16383,
+              "read-back: the parts hold every byte of any length");
 ReadBack g_read_back;
+
+bool pageable(const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return false;
+}
 
 // Copies `bytes` from device memory after the work queued on `st` and waits.
 cudaError_t read_back(void* dst, const void* src, size_t bytes, int device, cudaStream_t st) {
     std::unique_lock<std::mutex> lk(g_read_back.mu, std::defer_lock);
-    if (bytes >= ReadBack::MIN_BYTES && lk.try_lock() && !g_read_back.pinned) {
+    const bool slots = bytes >= ReadBack::MIN_BYTES && pageable(dst);
+    if (slots && lk.try_lock() && !g_read_back.pinned) {
         void* v = nullptr;
         if (cudaHostAlloc(&v, ReadBack::THREADS * 2 * ReadBack::CHUNK, cudaHostAllocPortable) == cudaSuccess)
             g_read_back.pinned = (char*)v;
         else
             cudaGetLastError();  // no pinned memory to be had: copy plainly
     }
-    if (bytes < ReadBack::MIN_BYTES || !lk.owns_lock() || !g_read_back.pinned) {
+    if (!lk.owns_lock() || !g_read_back.pinned) {
         const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
         return e != cudaSuccess ? e : cudaStreamSynchronize(st);
     }
-    const size_t part = (bytes / ReadBack::THREADS + 4095) & ~(size_t)4095;
+    const size_t part = ReadBack::part(bytes);
     std::atomic<int> error{cudaSuccess};
     auto work = [&](size_t t) {
         const size_t lo = std::min(bytes, t * part), hi = std::min(bytes, lo + part);
