@@ -61,6 +61,13 @@ int rt_session_destroy(rt_session* s);
 /* Message of the last failure on this thread ("" if none). */
 const char* rt_last_error(void);
 
+/* Gives back what the process keeps between calls and sessions: device memory
+ * that destroyed sessions have returned to the library's pool, and the 16 MB
+ * of pinned host memory through which results of 24 MB and more are read into
+ * pageable memory (made at the first such read). Sessions stay usable, and
+ * later calls take the memory anew. */
+int rt_release_memory(void);
+
 /* Render `count` more samples per pixel, sample indices
  * [sample_start, sample_start + count), adding them to the f64
  * accumulator. Replaces PtSession::render_samples / WfSession::render_samples

@@ -29,9 +29,15 @@ using namespace rt;
 
 namespace rt {
 
+namespace {
+struct {
+    std::mutex mu;
+    cudaMemPool_t pools[64] = {};
+} g_pools;
+}  // namespace
+
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st) {
-    static std::mutex mu;
-    static cudaMemPool_t pools[64] = {};
+    auto& [mu, pools] = g_pools;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -59,6 +65,14 @@ cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st) {
 }
 
 cudaError_t pool_free(void* p, cudaStream_t st) { return cudaFreeAsync(p, st); }
+
+cudaError_t pool_trim() {
+    std::lock_guard<std::mutex> lk(g_pools.mu);
+    cudaError_t e = cudaSuccess;
+    for (cudaMemPool_t pool : g_pools.pools)
+        if (pool && e == cudaSuccess) e = cudaMemPoolTrimTo(pool, 0);
+    return e;
+}
 
 }  // namespace rt
 
@@ -117,8 +131,8 @@ struct DeviceScope {
 // 4 KB. Large ones go through pinned slots instead, each of a few threads copying
 // its own part of the destination out of its own two slots while the next chunk
 // is in flight, so the faults and the copies run side by side. One 16 MB buffer,
-// made at the first large read-back and kept for the process; a call that finds
-// it taken copies plainly. A 961 x 541 film (37 MB) came back in 8.1 ms, now 3.6;
+// made at the first large read-back and kept until rt_release_memory or the end of
+// the process; a call that finds it taken copies plainly. A 961 x 541 film (37 MB) came back in 8.1 ms, now 3.6;
 // below 24 MB starting the threads costs more than they save (5.5 MB: 0.4 ms more,
 // 21 MB into pages in use 1.06 ms against 1.12; 27 MB 1.34 against 1.27).
 // Memory that CUDA knows (pinned, registered, managed) takes the plain copy, which
@@ -194,6 +208,18 @@ cudaError_t read_back(void* dst, const void* src, size_t bytes, int device, cuda
     for (size_t t = 0; t < made; t++) helpers[t].join();
     if (error.load() != cudaSuccess) cudaStreamSynchronize(st);  // nothing still writes the slots
     return (cudaError_t)error.load();
+}
+
+// The slots and the device pools' free blocks, returned to the system.
+cudaError_t release_memory() {
+    cudaError_t e = cudaSuccess;
+    {
+        std::lock_guard<std::mutex> lk(g_read_back.mu);  // a read-back in flight ends first
+        if (g_read_back.pinned) e = cudaFreeHost(g_read_back.pinned);
+        g_read_back.pinned = nullptr;
+    }
+    const cudaError_t t = pool_trim();
+    return e != cudaSuccess ? e : t;
 }
 
 // Waves of a slab at most: a bounce each, and the surfaces passed without one.
@@ -347,6 +373,11 @@ static void launch_shadow(rt_session* s, const Paths& P, const PtConsts& C, cuda
 extern "C" {
 
 const char* rt_last_error(void) { return g_err.c_str(); }
+
+int rt_release_memory(void) {
+    CUDA_TRY(release_memory());
+    return RT_OK;
+}
 
 int rt_session_create(const rt_scene_desc* scene, const rt_params* params, rt_session** out) {
     if (!out) return fail(RT_ERR_INVALID, "out is NULL");

@@ -33,7 +33,7 @@ EXPORTS = ("rt_session_create", "rt_session_destroy", "rt_last_error", "rt_rende
            "rt_average_spp", "rt_checkpoint_save_rckp", "rt_rckp_write", "rt_accum_exr_write",
            "rt_accum_exr_info", "rt_accum_exr_read", "rt_accum_merge", "rt_read_film", "rt_denoise",
            "rt_denoise_film", "rt_film_exr_write", "rt_pcg_streams", "rt_light_sample_batch",
-           "rt_light_pmf_batch", "rt_transmittance_batch", "rt_set_limits")
+           "rt_light_pmf_batch", "rt_transmittance_batch", "rt_set_limits", "rt_release_memory")
 
 
 class RtError(RuntimeError):
@@ -150,6 +150,11 @@ def hair_sample(params, wo, h, pixel, sample, n):
     _check(lib().rt_hair_sample(p.ctypes.data, w.ctypes.data, C.c_double(h), C.c_uint64(pixel), C.c_uint64(sample),
                                 C.c_uint64(n), out.ctypes.data))
     return out[:, :3], out[:, 3:6], out[:, 6]
+
+
+def release_memory():
+    """Gives back what the process keeps between sessions (rt_release_memory)."""
+    _check(lib().rt_release_memory())
 
 
 class PtSession:

@@ -69,3 +69,22 @@ def test_pinned_destinations_are_written_directly():
             assert np.array_equal(a, want)
             best.append(min(times))
     assert best[0] < 0.8 * best[1], best
+
+
+def test_release_memory_gives_back_and_leaves_sessions_usable():
+    """What destroyed sessions returned to the pool goes back to the driver; the pinned slots are made anew."""
+    keep = PtSession(scenes.cornell_box(64, 48), abi.make_params(max_depth=2, aovs=True))
+    with PtSession(scenes.cornell_box(1300, 900), abi.make_params(max_depth=2, aovs=True)) as g:
+        g.render_samples(0, 1)
+        _check(g)
+        held = g.stats()["device_bytes"]
+    free = torch.cuda.mem_get_info()[0]
+    backend.release_memory()
+    assert torch.cuda.mem_get_info()[0] - free > 0.5 * held > 1 << 20
+    backend.release_memory()
+    keep.render_samples(0, 1)
+    _check(keep)
+    keep.close()
+    with PtSession(scenes.cornell_box(1300, 900), abi.make_params(max_depth=2, aovs=True)) as g:
+        g.render_samples(0, 1)
+        _check(g)
