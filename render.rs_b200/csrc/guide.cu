@@ -998,10 +998,23 @@ int rt_guide_info(rt_guide* g, float* res_out, float* lo_out, float* inv_ext_out
     return 0;
 }
 
+// Whether a kernel may store to `p` itself: the forward pass writes 16 bytes at a
+// time, and only into memory of the device it runs on. A copy reaches whatever
+// CUDA can copy to (pinned or managed memory, another device's).
+static bool stores_reach(const void* p) {
+    cudaPointerAttributes a{};
+    int dev = 0;
+    if (((uintptr_t)p & 15u) || cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == dev;
+}
+
 int rt_guide_infer_device(rt_guide* g, const float* rec, uint32_t n, float* raw_out, void* stream) {
     if (!g || (n && (!rec || !raw_out))) return gfail(-1, "NULL argument");
     cudaStream_t st = (cudaStream_t)stream;
-    const bool direct = ((uintptr_t)raw_out & 15u) == 0;  // the kernel stores 16 bytes at a time
+    const bool direct = n && stores_reach(raw_out);
     int rc = launch_forward(g, rec, n, FWD_RAW, st, BatchSel{nullptr, 0, 1}, direct ? raw_out : nullptr);
     if (rc) return rc;
     if (n && !direct) G_TRY(cudaMemcpyAsync(raw_out, g->out, (size_t)n * G_OUT * 4, cudaMemcpyDeviceToDevice, st));

@@ -1,12 +1,14 @@
 """The training step's backward pass over batch sizes that fill one tile, several CTAs, all their tile pipelines and
 more than one tile per pipeline. Gradients are sums over records, so a batch's gradient is the sum of its chunks'
 (chunks of 1,000 use one pipeline per CTA and are checked against the f64 oracle in test_gpu_guide.py)."""
+import ctypes
 import zlib
 
 import numpy as np
 import pytest
 import torch
 
+from rtcuda import guide as guide_mod
 from rtcuda.guide import Guide, LEVELS, TABLE_ENTRIES
 
 pytestmark = pytest.mark.gpu
@@ -112,3 +114,25 @@ def test_training_gives_the_recorded_network():
     mlp, table = g.params()
     g.close()
     assert (zlib.crc32(mlp.tobytes()), zlib.crc32(table.tobytes())) == (1770624645, 2885379321)
+
+
+def test_inference_writes_any_memory_a_copy_reaches():
+    """Outputs in device memory of 16-byte and 4-byte alignment and in pinned host memory: the same values."""
+    g = Guide((-1, -1, -1), (1, 1, 1), seed=3)
+    n = 5000
+    rec = torch.from_numpy(_records(n, 4)).cuda()
+    want = g.infer(rec.cpu().numpy())
+    device = torch.zeros(n * 48 + 4, device="cuda")
+    pinned = torch.zeros(n * 48 + 4, pin_memory=True)
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for buf in (device, pinned):
+        for at in (0, 1, 4):
+            buf.zero_()
+            torch.cuda.synchronize()
+            guide_mod._check(guide_mod._g().rt_guide_infer_device(g.h, rec.data_ptr(), n, buf[at:].data_ptr(),
+                                                                  ctypes.c_void_p(st.cuda_stream)))
+            st.synchronize()
+            assert np.array_equal(buf[at:at + n * 48].cpu().numpy().reshape(n, 48), want)
+            assert (buf[:at] == 0).all() and (buf[at + n * 48:] == 0).all()
+    g.close()
