@@ -84,3 +84,27 @@ def test_small_meshes_build_alike(tris, presence):
     assert hit.sum() > 2000 and ((a[0] != 0xFFFFFFFF) == hit).mean() > 0.999
     both = hit & (a[0] != 0xFFFFFFFF)
     assert (np.abs(a[2][both] - ot[both]) <= 1e-4 * (1.0 + ot[both])).mean() > 0.999
+
+
+@pytest.mark.parametrize("offsets", [
+    [(0, 0, 0), (1, 0, 0)], [(1, 0, 0), (0, 0, 0)], [(0, 0, 0), (0, 0, 0)], [(0, 0, 0), (0, 0, 1e-7)],
+    [(0, 1e-13, 0), (0, 0, 0)], [(2, 1, 0), (0, 1, 2), (1, 1, 1)]])
+def test_pairs_part_alike(offsets):
+    """Two items left to part take no SAH sweep: either order along the widest axis, one place, centroids within f32 of
+    one another."""
+    s = Scene(8, 8)
+    mat = s.add_material(matte((0.5, 0.5, 0.5)))
+    cube = s.add_mesh(*scenes.unit_cube())
+    for at in offsets:
+        s.add_instance(cube, mat, affine(np.eye(3), at))
+    rays = scenes.triangle_cloud_rays(2048, seed=7)
+    rays[0, :, :3] *= 3.0
+    d = np.asarray(offsets)[np.arange(2048) % len(offsets)] - rays[0, :, :3]
+    rays[1, :, :3] = d / np.linalg.norm(d, axis=1, keepdims=True)
+    got = {}
+    for build in ("device", "host"):
+        with PtSession(s, abi.make_params(max_depth=4, max_paths=64, bvh_build=build)) as g:
+            got[build] = g.intersect(rays) + (g.stats()["tlas_nodes"],)
+    assert got["device"][3] == got["host"][3]
+    assert np.array_equal(got["device"][2], got["host"][2])
+    assert np.isfinite(got["host"][2]).all()
