@@ -108,3 +108,26 @@ def test_pairs_part_alike(offsets):
     assert got["device"][3] == got["host"][3]
     assert np.array_equal(got["device"][2], got["host"][2])
     assert np.isfinite(got["host"][2]).all()
+
+
+def test_large_mesh_instanced_densely():
+    """A BLAS and a TLAS whose host trees are collapsed on all threads, the instances split along the BLAS's second
+    level: the builders agree on the trees' sizes and on every hit."""
+    rng = np.random.default_rng(5)
+    s = Scene(8, 8)
+    mat = s.add_material(matte((0.5, 0.5, 0.5)))
+    mesh = s.add_mesh(*scenes.triangle_cloud_mesh(150_000, seed=9))
+    at = rng.normal(size=(1500, 3)) * 0.1
+    rot = scenes.random_rotations(rng, len(at))
+    for k in range(len(at)):
+        s.add_instance(mesh, mat, affine(rot[k], at[k]))
+    rays = scenes.triangle_cloud_rays(2048, seed=7)
+    got = {}
+    for build in ("device", "host"):
+        with PtSession(s, abi.make_params(max_depth=4, max_paths=64, bvh_build=build)) as g:
+            st = g.stats()
+            got[build] = g.intersect(rays) + (st["blas_nodes"], st["tlas_nodes"])
+    a, b = got["device"], got["host"]
+    assert a[3:] == b[3:] and a[3] > 16_384 and a[4] > 16_384
+    assert np.array_equal(a[2], b[2])
+    assert np.isfinite(a[2]).mean() > 0.5
