@@ -274,19 +274,23 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) k_guide_fwd(GuideDev G, const 
 }
 
 // ---- backward -----------------------------------------------------------------
-// One CTA per SM runs BWD_GROUPS tile pipelines (one warpgroup and one tile
-// each) over weights they share. Per layer a pipeline stores dZ and the layer's
-// input H once, row by row in the core-matrix layout, H with a column of ones
-// after its last input, and issues both GEMMs on them: dH = dZ W reads dZ
-// K-major, [dW | db]^T = [H | 1]^T dZ reads H and dZ transposed (MN-major
+// One persistent CTA per SM runs BWD_GROUPS tile pipelines (one warpgroup each),
+// a tile each per round, over weights they share. Per layer a pipeline stores dZ
+// and the layer's input H once, row by row in the core-matrix layout, H with a
+// column of ones after its last input, and issues both GEMMs on them: dH = dZ W
+// reads dZ K-major, [dW | db]^T = [H | 1]^T dZ reads H and dZ transposed (MN-major
 // descriptors over the same bytes), so nothing is copied transposed and the
 // bias gradients fall out as one more row. With M = 128 that GEMM also reads
 // columns past the ones (bytes of the next rows, or past the end of the
 // buffer): accumulator rows nobody reads. A lane of the accumulator holds an
 // input, so a warp's stores to the row-major partial row are neighbours.
-// Every tile's sums go to a row of their own. The sum over tiles keeps one
-// fixed order whatever the launch shape (k_guide_grad_reduce), so a network
-// trained on the same records stays the same bit for bit.
+// The sum over tiles keeps one fixed order whatever the launch shape, so a network
+// trained on the same records stays the same bit for bit: row r of `half` (two per
+// SM) adds tiles r, r + half, r + 2 half, ... in turn, then the rows are added in
+// turn, all in f32. Pipeline p takes tile p of each round of 2 half tiles. Those
+// below `half` keep row p. The others write their round's tile to a row of its own,
+// which the pipeline half places below, in the same CTA, adds a round later
+// (two sets of these rows, used in turn); k_guide_grad_reduce adds the last.
 // The pass is latency-bound (a chain of four GEMM pairs per tile, nothing near a
 // peak): transposed copies of dZ and H written two bytes at a time, row-strided
 // global sums and two one-tile CTAs per SM took 186 us for 65,536 records; with
@@ -300,20 +304,21 @@ constexpr uint32_t B_HCOLS = 72, B_GROUP = 16384 + TILE * B_HCOLS * 2;
 constexpr int B_ACT = F_ACT, B_BYTES = B_ACT + BWD_GROUPS * B_GROUP + 1024;
 static_assert(BWD_TMEM_COLS == 512, "backward: TMEM allocation is a power of two");
 // The GEMM over H reads 16 blocks of 8 columns for each 8 rows.
-static_assert((TILE / 8 - 1) * B_HCOLS * 16 + 16 * 128 <= TILE * B_HCOLS * 2 + 1024, "backward: reads past H stay inside");
+static_assert((TILE / 8 - 1) * B_HCOLS * 16 + 16 * 128 <= TILE * B_HCOLS * 2 + 1024,
+              "backward: reads past H stay inside");
 
-// Tiles [tile0, tile0 + BWD_GROUPS * gridDim.x), one per pipeline; pipeline p
-// writes partial row p. Rows below `half` go on summing what an earlier launch
-// of the same batch left there (fresh: the first launch).
+// ROUNDS: there may be more than one (the loop and the sums of earlier rounds cost
+// a batch of one round 8 us of 34).
+template <bool ROUNDS>
 __global__ void __launch_bounds__(BWD_THREADS, 1) k_guide_bwd(GuideDev G, const __nv_bfloat16* __restrict__ X0,
                                                               const __nv_bfloat16* __restrict__ acts,
                                                               const float* __restrict__ out,
                                                               const float* __restrict__ rec, uint32_t n, BatchSel B,
-                                                              uint32_t tile0, uint32_t half, float* part, float* dX0,
-                                                              float* loss_sum, uint32_t* err) {
+                                                              uint32_t half, float* part, float* dX0, float* loss_sum,
+                                                              uint32_t* err) {
     uint32_t begin;
     n = batch_slice(B, n, begin);
-    if ((uint64_t)(tile0 + blockIdx.x) * TILE >= n) return;  // no tile for this CTA
+    if ((uint64_t)blockIdx.x * TILE >= n) return;  // no tile for this CTA
     rec += 16 * (size_t)begin;
     extern __shared__ __align__(1024) uint8_t sm[];
     __shared__ uint64_t mbar[BWD_GROUPS];
@@ -339,120 +344,131 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_guide_bwd(GuideDev G, const 
     const uint32_t acc = tmem_base + 128u * grp;
     const uint32_t lane_addr = acc + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t s0 = smem_u32(sm);
-    const uint32_t pipe = grp * gridDim.x + blockIdx.x, tile = tile0 + pipe;
-    float* gW = part + (size_t)pipe * G_NPARAMS;
-    float* gb = gW + G_NWEIGHTS;
-    const bool fresh = tile0 == 0 || pipe >= half;
+    const uint32_t pipe = grp * gridDim.x + blockIdx.x, tiles = (n + TILE - 1) / TILE;
     uint32_t phase = 0;
     float loss = 0.f;
-    if ((uint64_t)tile * TILE < n) {
-        const uint32_t row = tile * TILE + gt;
-        const bool valid = row < n;
-        float dz[64];
-        if (valid) {
-            float o[G_OUT];
-            const float4* op = reinterpret_cast<const float4*>(out + (size_t)row * G_OUT);
+    for (uint32_t round = 0; round == 0 || (ROUNDS && round * 2 * half + blockIdx.x < tiles); round++) {
+        const uint32_t tile = round * 2 * half + pipe, set = half * (round & 1u);
+        float* gW = part + (size_t)(pipe < half ? pipe : pipe + set) * G_NPARAMS;
+        // The row of the tile half places on in the round before.
+        const size_t upper = (size_t)(2 * half - set) * G_NPARAMS;
+        const bool add = ROUNDS && round > 0 && pipe < half;
+        if (tile < tiles && !group_failed[grp]) {
+            const uint32_t row = tile * TILE + gt;
+            const bool valid = row < n;
+            float dz[64];
+            if (valid) {
+                float o[G_OUT];
+                const float4* op = reinterpret_cast<const float4*>(out + (size_t)row * G_OUT);
 #pragma unroll
-            for (int c = 0; c < G_OUT / 4; c++) {
-                float4 q = op[c];
-                o[4 * c] = q.x;
-                o[4 * c + 1] = q.y;
-                o[4 * c + 2] = q.z;
-                o[4 * c + 3] = q.w;
+                for (int c = 0; c < G_OUT / 4; c++) {
+                    float4 q = op[c];
+                    o[4 * c] = q.x;
+                    o[4 * c + 1] = q.y;
+                    o[4 * c + 2] = q.z;
+                    o[4 * c + 3] = q.w;
+                }
+                const float* r = rec + 16 * (size_t)row;
+                loss += mixture_loss_grad(o, f3(r[9], r[10], r[11]), r[12], dz);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 64; k++) dz[k] = 0.f;
             }
-            const float* r = rec + 16 * (size_t)row;
-            loss += mixture_loss_grad(o, f3(r[9], r[10], r[11]), r[12], dz);
-        } else {
 #pragma unroll
-            for (int k = 0; k < 64; k++) dz[k] = 0.f;
-        }
+            for (int l = 3; l >= 0; l--) {
+                const int K_in = l_in(l), N_out = l_out(l);
+                // dZ and the layer input H, rows of this tile. H keeps its row
+                // length in every layer: with another stride in layer 0 a thread's
+                // row would land on rows whose ReLU masks others still read.
 #pragma unroll
-        for (int l = 3; l >= 0; l--) {
-            const int K_in = l_in(l), N_out = l_out(l);
-            // dZ and the layer input H, rows of this tile. H keeps its row
-            // length in every layer: with another stride in layer 0 a thread's
-            // row would land on rows whose ReLU masks others still read.
+                for (int c = 0; c < 8; c++)
+                    if (8 * c < N_out)
+                        *reinterpret_cast<uint4*>(sm + dz_off + core_offset(gt, 8 * c, N_out)) =
+                            make_uint4(pack_bf16(dz[8 * c], dz[8 * c + 1]), pack_bf16(dz[8 * c + 2], dz[8 * c + 3]),
+                                       pack_bf16(dz[8 * c + 4], dz[8 * c + 5]),
+                                       pack_bf16(dz[8 * c + 6], dz[8 * c + 7]));
+                const uint4* hp = l > 0 ? reinterpret_cast<const uint4*>(acts + ((size_t)row * 3 + (l - 1)) * G_HID)
+                                        : reinterpret_cast<const uint4*>(X0 + (size_t)row * G_IN);
 #pragma unroll
-            for (int c = 0; c < 8; c++)
-                if (8 * c < N_out)
-                    *reinterpret_cast<uint4*>(sm + dz_off + core_offset(gt, 8 * c, N_out)) =
-                        make_uint4(pack_bf16(dz[8 * c], dz[8 * c + 1]), pack_bf16(dz[8 * c + 2], dz[8 * c + 3]),
-                                   pack_bf16(dz[8 * c + 4], dz[8 * c + 5]), pack_bf16(dz[8 * c + 6], dz[8 * c + 7]));
-            const uint4* hp = l > 0 ? reinterpret_cast<const uint4*>(acts + ((size_t)row * 3 + (l - 1)) * G_HID)
-                                    : reinterpret_cast<const uint4*>(X0 + (size_t)row * G_IN);
-#pragma unroll
-            for (int c = 0; c < 8; c++)
-                if (8 * c < K_in)
-                    *reinterpret_cast<uint4*>(sm + h_off + core_offset(gt, 8 * c, B_HCOLS)) =
-                        valid ? hp[c] : make_uint4(0, 0, 0, 0);
-            if (l == 0) *reinterpret_cast<uint4*>(sm + h_off + core_offset(gt, G_IN, B_HCOLS)) = ones;
-            fence_proxy_async_smem();
-            group_sync(grp);
-            if (gt == 0) {
+                for (int c = 0; c < 8; c++)
+                    if (8 * c < K_in)
+                        *reinterpret_cast<uint4*>(sm + h_off + core_offset(gt, 8 * c, B_HCOLS)) =
+                            valid ? hp[c] : make_uint4(0, 0, 0, 0);
+                if (l == 0) *reinterpret_cast<uint4*>(sm + h_off + core_offset(gt, G_IN, B_HCOLS)) = ones;
+                fence_proxy_async_smem();
+                group_sync(grp);
+                if (gt == 0) {
+                    tc_fence_after();
+                    const uint32_t w = s0 + (l == 0 ? F_W0 : l == 1 ? F_W1 : l == 2 ? F_W2 : F_W3);
+                    // dH[m][k] = sum_n dZ[m][n] W[n][k]  (N = K_in, K = N_out)
+                    tc_gemm_issue_ops(acc + 64u, umma_k_major(s0 + dz_off, N_out), umma_transposed(w, K_in), K_in,
+                                      N_out);
+                    // dW[n][k] = sum_m dZ[m][n] H[m][k], row k of the accumulator; row K_in: db
+                    tc_gemm_issue_ops(acc, umma_transposed(s0 + h_off, B_HCOLS), umma_transposed(s0 + dz_off, N_out),
+                                      N_out, TILE);
+                    tc_commit(&mbar[grp]);
+                }
+                if (!mbar_wait_or_drain(&mbar[grp], phase, G.wait_polls)) group_failed[grp] = 1;
+                phase ^= 1u;
+                group_sync(grp);
+                if (group_failed[grp]) break;
                 tc_fence_after();
-                const uint32_t w = s0 + (l == 0 ? F_W0 : l == 1 ? F_W1 : l == 2 ? F_W2 : F_W3);
-                // dH[m][k] = sum_n dZ[m][n] W[n][k]  (N = K_in, K = N_out)
-                tc_gemm_issue_ops(acc + 64u, umma_k_major(s0 + dz_off, N_out), umma_transposed(w, K_in), K_in, N_out);
-                // dW[n][k] = sum_m dZ[m][n] H[m][k], row k of the accumulator; row K_in: db
-                tc_gemm_issue_ops(acc, umma_transposed(s0 + h_off, B_HCOLS), umma_transposed(s0 + dz_off, N_out),
-                                  N_out, TILE);
-                tc_commit(&mbar[grp]);
-            }
-            if (!mbar_wait_or_drain(&mbar[grp], phase, G.wait_polls)) group_failed[grp] = 1;
-            phase ^= 1u;
-            group_sync(grp);
-            if (group_failed[grp]) break;
-            tc_fence_after();
-            if (gt < (l > 0 ? 96 : 64)) {  // whole warps: the inputs' lanes and the one after them, with the biases
-                float* at = gt < K_in ? gW + w_off(l) + gt : gb + b_off(l);
-                const int step = gt < K_in ? K_in : 1;
+                if (gt < (l > 0 ? 96 : 64)) {  // whole warps: the inputs' lanes and the one after them, with the biases
+                    float* at = gt < K_in ? gW + w_off(l) + gt : gW + G_NWEIGHTS + b_off(l);
+                    const int step = gt < K_in ? K_in : 1;
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    uint32_t r[32];
-                    tmem_ld32(lane_addr + 32 * h, r);
-                    if (gt <= K_in) {
+                    for (int h = 0; h < 2; h++) {
+                        uint32_t r[32];
+                        tmem_ld32(lane_addr + 32 * h, r);
+                        if (gt <= K_in) {
+                            // All loads, then all stores: the compiler cannot tell their rows apart.
+                            if (add)
 #pragma unroll
-                        for (int k = 0; k < 32; k++)
-                            if (32 * h + k < N_out) {
-                                const float v = __uint_as_float(r[k]);
-                                float* p = at + (32 * h + k) * step;
-                                *p = fresh ? v : *p + v;
-                            }
-                    }
-                    __syncwarp();
-                }
-            }
+                                for (int k = 0; k < 32; k++)
+                                    if (32 * h + k < N_out) {
+                                        const float* p = at + (32 * h + k) * step;
+                                        r[k] = __float_as_uint(*p + p[upper] + __uint_as_float(r[k]));
+                                    }
 #pragma unroll
-            for (int h = 0; h < (l > 0 ? 2 : 1); h++) {
-                uint32_t r[32];
-                tmem_ld32(lane_addr + 64 + 32 * h, r);
-                if (l > 0) {
-                    // dZ of the layer below: dH where its ReLU passed (its bf16
-                    // activations are positive unless the bits are zero).
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        const uint4 q =
-                            *reinterpret_cast<const uint4*>(sm + h_off + core_offset(gt, 32 * h + 8 * c, B_HCOLS));
-                        const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const int k = 8 * c + 2 * e;
-                            dz[32 * h + k] = (w4[e] & 0x7FFFu) ? __uint_as_float(r[k]) : 0.f;
-                            dz[32 * h + k + 1] = (w4[e] & 0x7FFF0000u) ? __uint_as_float(r[k + 1]) : 0.f;
+                            for (int k = 0; k < 32; k++)
+                                if (32 * h + k < N_out) at[(32 * h + k) * step] = __uint_as_float(r[k]);
                         }
+                        __syncwarp();
                     }
-                } else if (valid) {
-                    float4* d = reinterpret_cast<float4*>(dX0 + (size_t)row * 32);
-#pragma unroll
-                    for (int c = 0; c < 8; c++)
-                        d[c] = make_float4(__uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]),
-                                           __uint_as_float(r[4 * c + 2]), __uint_as_float(r[4 * c + 3]));
                 }
+#pragma unroll
+                for (int h = 0; h < (l > 0 ? 2 : 1); h++) {
+                    uint32_t r[32];
+                    tmem_ld32(lane_addr + 64 + 32 * h, r);
+                    if (l > 0) {
+                        // dZ of the layer below: dH where its ReLU passed (its bf16
+                        // activations are positive unless the bits are zero).
+#pragma unroll
+                        for (int c = 0; c < 4; c++) {
+                            const uint4 q =
+                                *reinterpret_cast<const uint4*>(sm + h_off + core_offset(gt, 32 * h + 8 * c, B_HCOLS));
+                            const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                const int k = 8 * c + 2 * e;
+                                dz[32 * h + k] = (w4[e] & 0x7FFFu) ? __uint_as_float(r[k]) : 0.f;
+                                dz[32 * h + k + 1] = (w4[e] & 0x7FFF0000u) ? __uint_as_float(r[k + 1]) : 0.f;
+                            }
+                        }
+                    } else if (valid) {
+                        float4* d = reinterpret_cast<float4*>(dX0 + (size_t)row * 32);
+#pragma unroll
+                        for (int c = 0; c < 8; c++)
+                            d[c] = make_float4(__uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]),
+                                               __uint_as_float(r[4 * c + 2]), __uint_as_float(r[4 * c + 3]));
+                    }
+                }
+                __syncwarp();
+                tc_fence_before();
             }
-            __syncwarp();
-            tc_fence_before();
+            if (gt == 0 && group_failed[grp]) atomicOr(err, GERR_WAIT);
         }
-        if (gt == 0 && group_failed[grp]) atomicOr(err, GERR_WAIT);
+        if (ROUNDS) __syncthreads();  // this round's rows are written, those of the round before read
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, off);
@@ -470,34 +486,21 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_guide_bwd(GuideDev G, const 
     }
 }
 
-// The gradient's order of summation: row r of `half` (two per SM) adds tiles r,
-// r + half, r + 2 half, ... in turn, then the rows are added in turn, all in
-// f32. A launch of the backward pass leaves tiles tile0 + r and tile0 + half + r
-// in rows r and half + r, so a batch of several launches folds the upper rows
-// into the lower ones between them.
-__global__ void __launch_bounds__(256) k_guide_grad_fold(float* part, uint32_t n, BatchSel B, uint32_t tile0,
-                                                         uint32_t half) {
-    uint32_t begin;
-    n = batch_slice(B, n, begin);
-    const uint32_t i = blockIdx.x * 256 + threadIdx.x, r = blockIdx.y;
-    if (i >= (uint32_t)G_NPARAMS || (uint64_t)(tile0 + half + r) * TILE >= n) return;
-    part[(size_t)r * G_NPARAMS + i] += part[(size_t)(half + r) * G_NPARAMS + i];
-}
-
-// Adds the rows of the last launch (its first tile: tile0) to the MLP gradient.
+// Adds the rows to the MLP gradient in turn, each with the tile that its pipeline
+// did not get to add (a row's last tile, where the upper pipelines took it).
 // Sixteen warps a block bring 32 parameters' rows to shared memory, all loads
 // in flight together, and one warp adds them in order. Rows of a failed
 // backward pass are left out.
 constexpr int GR_PARAMS = 32, GR_SLICES = 16, GR_ROWS = 304;
 __global__ void __launch_bounds__(GR_PARAMS* GR_SLICES) k_guide_grad_reduce(const float* __restrict__ part, uint32_t n,
-                                                                            BatchSel B, uint32_t tile0, uint32_t half,
-                                                                            float* gw,
+                                                                            BatchSel B, uint32_t half, float* gw,
                                                                             const uint32_t* __restrict__ err) {
     __shared__ float row[GR_ROWS][GR_PARAMS];
     uint32_t begin;
     n = batch_slice(B, n, begin);
     if (*err) return;
     const uint32_t tiles = (n + TILE - 1) / TILE, rows = min(tiles, half);
+    const uint32_t round = tiles ? (tiles - 1) / (2 * half) : 0u, rem = tiles - round * 2 * half;  // the last round
     const uint32_t c = threadIdx.x % GR_PARAMS, sl = threadIdx.x / GR_PARAMS;
     const uint32_t i = blockIdx.x * GR_PARAMS + c;
     const bool own = i < (uint32_t)G_NPARAMS;
@@ -508,9 +511,11 @@ __global__ void __launch_bounds__(GR_PARAMS* GR_SLICES) k_guide_grad_reduce(cons
 #pragma unroll
         for (int k = 0; k < GR_ROWS / GR_SLICES; k++) {
             const uint32_t r = r0 + k * GR_SLICES + sl;
-            const bool in = own && r < rows, pair = in && tile0 + half + r < tiles;
+            const bool in = own && r < rows;
+            const uint32_t last = r < rem ? round : round - 1u;  // the row's last round
+            const bool pair = in && (r >= rem || half + r < rem);
             lower[k] = in ? part[(size_t)r * G_NPARAMS + i] : 0.f;
-            upper[k] = pair ? part[(size_t)(half + r) * G_NPARAMS + i] : 0.f;
+            upper[k] = pair ? part[(size_t)(half + half * (last & 1u) + r) * G_NPARAMS + i] : 0.f;
         }
 #pragma unroll
         for (int k = 0; k < GR_ROWS / GR_SLICES; k++) row[k * GR_SLICES + sl][c] = lower[k] + upper[k];
@@ -700,7 +705,7 @@ struct rt_guide {
     __nv_bfloat16* w16 = nullptr;
     float* t32 = nullptr;      // table master (levels * T * 2)
     unsigned long long* gt = nullptr;  // table gradient, 2^-24 fixed point
-    float* part = nullptr;     // a launch's tiles' dW / db (sms x BWD_GROUPS rows of G_NPARAMS)
+    float* part = nullptr;     // dW / db rows of the backward pipelines (3/2 BWD_GROUPS per SM, of G_NPARAMS)
     float* mt = nullptr;
     float* vt = nullptr;
     __half* t16 = nullptr;
@@ -788,15 +793,14 @@ static int launch_backward(rt_guide* g, const float* rec, uint32_t n, cudaStream
     uint32_t tiles = (n + TILE - 1) / TILE;
     const uint32_t sms = (uint32_t)g->sms, half = BWD_GROUPS / 2 * sms;
     G_TRY(cudaMemsetAsync(g->loss, 0, 4, st));
-    uint32_t tile0 = 0;
-    for (;; tile0 += 2 * half) {
-        k_guide_bwd<<<std::min(tiles - tile0, sms), BWD_THREADS, B_BYTES, st>>>(
-            g->G, g->X0, g->acts, g->out, rec, n, B, tile0, half, g->part, g->dX0, g->loss, g->err);
-        if (tiles - tile0 <= 2 * half) break;
-        k_guide_grad_fold<<<dim3((G_NPARAMS + 255) / 256, half), 256, 0, st>>>(g->part, n, B, tile0, half);
-    }
+    if (tiles <= 2 * half)
+        k_guide_bwd<false><<<std::min(tiles, sms), BWD_THREADS, B_BYTES, st>>>(g->G, g->X0, g->acts, g->out, rec, n, B,
+                                                                           half, g->part, g->dX0, g->loss, g->err);
+    else
+        k_guide_bwd<true><<<sms, BWD_THREADS, B_BYTES, st>>>(g->G, g->X0, g->acts, g->out, rec, n, B, half, g->part,
+                                                             g->dX0, g->loss, g->err);
     k_guide_grad_reduce<<<(G_NPARAMS + GR_PARAMS - 1) / GR_PARAMS, GR_PARAMS * GR_SLICES, 0, st>>>(
-        g->part, n, B, tile0, half, g->gw, g->err);
+        g->part, n, B, half, g->gw, g->err);
     k_guide_hash_bwd<<<(n + HB_WARPS - 1) / HB_WARPS, 32 * HB_WARPS, 0, st>>>(g->G, rec, g->dX0, n, B, g->gt);
     G_TRY(cudaGetLastError());
     return 0;
@@ -880,7 +884,7 @@ int rt_guide_create(const float* lo, const float* hi, uint64_t seed, float lr, r
     rc = rc ? rc : g->alloc(&g->w16, G_NWEIGHTS);
     rc = rc ? rc : g->alloc(&g->t32, tn);
     rc = rc ? rc : g->alloc(&g->gt, tn);
-    rc = rc ? rc : g->alloc(&g->part, (size_t)g->sms * BWD_GROUPS * G_NPARAMS);
+    rc = rc ? rc : g->alloc(&g->part, (size_t)g->sms * BWD_GROUPS / 2 * 3 * G_NPARAMS);
     rc = rc ? rc : g->alloc(&g->mt, tn);
     rc = rc ? rc : g->alloc(&g->vt, tn);
     rc = rc ? rc : g->alloc(&g->t16, tn);
@@ -896,7 +900,8 @@ int rt_guide_create(const float* lo, const float* hi, uint64_t seed, float lr, r
     cudaFuncSetAttribute(k_guide_fwd<FWD_RAW>, cudaFuncAttributeMaxDynamicSharedMemorySize, F_BYTES);
     cudaFuncSetAttribute(k_guide_fwd<FWD_TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, F_BYTES);
     cudaFuncSetAttribute(k_guide_fwd<FWD_RENDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, F_BYTES);
-    cudaFuncSetAttribute(k_guide_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, B_BYTES);
+    cudaFuncSetAttribute(k_guide_bwd<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, B_BYTES);
+    cudaFuncSetAttribute(k_guide_bwd<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, B_BYTES);
     cudaFuncSetAttribute(k_tc_selftest, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
     // Init: He-uniform weights, zero biases; table U(-1e-4, 1e-4) (instant-ngp).
     std::mt19937_64 rng(seed);

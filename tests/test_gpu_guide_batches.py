@@ -62,8 +62,8 @@ def test_training_is_reproducible():
 @pytest.mark.parametrize("n", [5, 300 * 128 + 77, 592 * 128, 592 * 128 + 1, 1500 * 128 + 5])
 def test_gradient_keeps_its_order_of_summation(n):
     """Row r of two per SM adds tiles (128 records) r, r + rows, r + 2 rows, ... in turn, then the rows are added in
-    turn, in f32: bit for bit what the tiles' own gradients give in that order, over batches of one launch of the
-    backward pass, its limit and several."""
+    turn, in f32: bit for bit what the tiles' own gradients give in that order, over batches of one round of the
+    backward pass's pipelines, exactly that, and several."""
     g = Guide((-1, -1, -1), (1, 1, 1), seed=3)
     rec = _records(n, n)
     tiles = [g.grads(rec[k:k + 128], table=False)[2] for k in range(0, n, 128)]
