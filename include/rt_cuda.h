@@ -281,6 +281,12 @@ int rt_read_film(rt_session* s, float* film);
 int rt_denoise(rt_session* s, float* rgb);
 int rt_denoise_film(const float* film, uint32_t width, uint32_t height, float* rgb);
 
+/* Diagnostic: the median positive depth as the denoiser selects it on the
+ * device (src/output/denoise.rs:56-64: the element at count / 2 in ascending
+ * order of the positive ones among depth[0..n)), 0 when none is positive.
+ * Runs on the current device. */
+int rt_depth_median(const float* depth, uint32_t n, float* median);
+
 /* A film as the reference's multilayer EXR (src/output/multilayer.rs:
  * channels R G B, diffuse.*, specular.*, albedo.*, N.*, depth.Z, id.x,
  * id.coverage in name order; layer "rgba"; the id manifest "id:name;..." in

@@ -21,6 +21,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -80,8 +81,7 @@ __global__ void k_denoise_prep(const float* __restrict__ film, uint32_t npix, fl
 // to the host and selecting there took 4 ms of a 961 x 541 film.
 struct DepthSelect {
     uint32_t hist[2048];
-    uint32_t prefix, rank;  // bits fixed so far (in place), rank among the depths that have them
-    uint32_t any;           // some depth is positive
+    uint32_t prefix, rank;  // bits fixed so far (in place; all ones when no depth is positive), rank among those
     float inv_scale;        // 1 / max(median, 1e-3), the median 1 when there is none
 };
 
@@ -230,6 +230,20 @@ int film_decode_device(const double* accum, const float* aux, uint32_t npix, flo
     return RT_OK;
 }
 
+// Fills `sel` with the median positive depth (guide w) of npix pixels.
+static cudaError_t select_median_depth(const float4* guide, uint32_t npix, DepthSelect* sel, cudaStream_t st) {
+    const cudaError_t e = cudaMemsetAsync(sel, 0, sizeof(DepthSelect), st);
+    if (e != cudaSuccess) return e;
+    const int hb = (int)std::min<uint32_t>((npix + FB - 1) / FB, 592);  // four blocks per SM
+    k_depth_hist<0><<<hb, FB, 0, st>>>(guide, npix, sel);
+    k_depth_pick<0><<<1, 1024, 0, st>>>(sel);
+    k_depth_hist<1><<<hb, FB, 0, st>>>(guide, npix, sel);
+    k_depth_pick<1><<<1, 1024, 0, st>>>(sel);
+    k_depth_hist<2><<<hb, FB, 0, st>>>(guide, npix, sel);
+    k_depth_pick<2><<<1, 1024, 0, st>>>(sel);
+    return cudaGetLastError();
+}
+
 // Denoise a device film into device rgb (3 floats per pixel) on `st`, without
 // waiting for it.
 int denoise_device(const float* film, uint32_t w, uint32_t h, float* rgb, cudaStream_t st) {
@@ -247,14 +261,7 @@ int denoise_device(const float* film, uint32_t w, uint32_t h, float* rgb, cudaSt
     // Depth scale: the median positive depth (denoise.rs:56-64).
     DepthSelect* sel;
     FM_TRY(B.get(&sel, 1));
-    FM_TRY(cudaMemsetAsync(sel, 0, sizeof(DepthSelect), st));
-    const int hb = (int)std::min<uint32_t>((npix + FB - 1) / FB, 592);  // four blocks per SM
-    k_depth_hist<0><<<hb, FB, 0, st>>>(guide, npix, sel);
-    k_depth_pick<0><<<1, 1024, 0, st>>>(sel);
-    k_depth_hist<1><<<hb, FB, 0, st>>>(guide, npix, sel);
-    k_depth_pick<1><<<1, 1024, 0, st>>>(sel);
-    k_depth_hist<2><<<hb, FB, 0, st>>>(guide, npix, sel);
-    k_depth_pick<2><<<1, 1024, 0, st>>>(sel);
+    FM_TRY(select_median_depth(guide, npix, sel, st));
     float sigma = 8.0f;
     dim3 grid((w + 15) / 16, (h + 15) / 16);
     int cur = 0;
@@ -296,6 +303,37 @@ extern "C" int rt_denoise_film(const float* film, uint32_t width, uint32_t heigh
     }
     const cudaError_t done = cudaStreamSynchronize(st);
     if (!rc && done != cudaSuccess) rc = fail_film(RT_ERR_CUDA, std::string("denoise: ") + cudaGetErrorString(done));
+    cudaStreamDestroy(st);
+    return rc;
+}
+
+extern "C" int rt_depth_median(const float* depth, uint32_t n, float* median) {
+    if ((n && !depth) || !median) return fail_film(RT_ERR_INVALID, "NULL argument");
+    *median = 0.0f;
+    if (n == 0) return RT_OK;
+    cudaStream_t st;
+    FM_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    int rc = RT_OK;
+    {
+        Bufs B(st);
+        float4* guide = nullptr;
+        DepthSelect* sel = nullptr;
+        uint32_t bits = 0xFFFFFFFFu;
+        cudaError_t e = B.get(&guide, n);
+        if (e == cudaSuccess) e = B.get(&sel, 1);
+        std::vector<float4> g(n);
+        for (uint32_t i = 0; i < n; i++) g[i].w = depth[i];
+        if (e == cudaSuccess) e = cudaMemcpyAsync(guide, g.data(), 16ull * n, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = select_median_depth(guide, n, sel, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&bits, &sel->prefix, 4, cudaMemcpyDeviceToHost, st);
+        const cudaError_t done = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) e = done;
+        if (e != cudaSuccess)
+            rc = fail_film(e == cudaErrorMemoryAllocation ? RT_ERR_OOM : RT_ERR_CUDA, cudaGetErrorString(e));
+        else if (bits != 0xFFFFFFFFu)
+            memcpy(median, &bits, 4);
+    }
+    cudaStreamSynchronize(st);
     cudaStreamDestroy(st);
     return rc;
 }

@@ -33,7 +33,7 @@ EXPORTS = ("rt_session_create", "rt_session_destroy", "rt_last_error", "rt_rende
            "rt_average_spp", "rt_checkpoint_save_rckp", "rt_rckp_write", "rt_accum_exr_write",
            "rt_accum_exr_info", "rt_accum_exr_read", "rt_accum_merge", "rt_read_film", "rt_denoise",
            "rt_denoise_film", "rt_film_exr_write", "rt_pcg_streams", "rt_light_sample_batch",
-           "rt_light_pmf_batch", "rt_transmittance_batch", "rt_set_limits", "rt_release_memory")
+           "rt_light_pmf_batch", "rt_transmittance_batch", "rt_set_limits", "rt_release_memory", "rt_depth_median")
 
 
 class RtError(RuntimeError):
@@ -374,6 +374,14 @@ def film_array(film):
     for k, (o, n) in FILM_LAYERS.items():
         a[..., o:o + n] = np.asarray(film[k], dtype=np.float32).reshape(h, w, -1)[..., :n]
     return a
+
+
+def depth_median(depth):
+    """The denoiser's depth scale before its lower bound (rt_depth_median): the median positive depth, 0 for none."""
+    d = np.ascontiguousarray(depth, dtype=np.float32).reshape(-1)
+    out = C.c_float()
+    _check(lib().rt_depth_median(d.ctypes.data, len(d), C.byref(out)))
+    return np.float32(out.value)
 
 
 def denoise_film(film):
