@@ -781,11 +781,14 @@ __device__ __forceinline__ void ray_pump(const DevScene& S, uint32_t n, uint32_t
 // (leaf_coop, PRES) instead of by the shade kernel's skip waves.
 // QUAD: the scene has quadrics or curve sets; MOT: motion blur (rays carry
 // their path's shutter time; launched with QUAD).
-// BLOCKS: resident blocks per SM. Six leave 80 registers (28 bytes spill), which
-// pays where rays wait for nodes from L2: with RT_EXTEND_LARGE nodes and more the
-// closest hits of the cloud's frame take 11.0 ms instead of 11.4 and of the
-// instanced scene's 15.2 instead of 15.8. Scenes of a few nodes find them in L1
-// and lose with six (Cornell 0.90 -> 0.94 ms), so they keep five.
+// BLOCKS: resident blocks per SM. Six leave 80 registers (a few bytes spill), which
+// pays where rays walk far and wait for nodes. On clouds of one mesh the closest
+// hits of a frame take, with five and six: at 2,640 nodes 3.30 and 3.29 ms, at 4,510
+// 4.27 and 4.21, at 34,186 5.33 and 5.22; the 1M-triangle cloud 11.4 and 11.0, the
+// materials' 1,000 instances 15.8 and 15.2. Short walks lose 2-4% with six: clouds
+// below 2,000 nodes 1%, Cornell 0.90 and 0.94 ms, and a scene of 10,000 nodes in a
+// few instances 0.72 and 0.75 ms. The number of nodes stands in for the length of
+// the walks, which is not known before the launch.
 #define RT_EXTEND_LARGE 4096u
 template <int BLOCK, bool PRES, bool QUAD = false, bool MOT = false, int BLOCKS = RT_TRAV_MIN_BLOCKS>
 __global__ void __launch_bounds__(BLOCK, BLOCKS) k_extend(DevScene S, Paths P, uint32_t qsel) {
@@ -1049,9 +1052,11 @@ __device__ __forceinline__ float light_pdf_sa(const DevLight& L, float3 origin, 
     return 0.0f;
 }
 
-// Four resident blocks: 124 registers without spills, where the compiler's own
-// choice of 140 left three (materials 1080p x 6 spp: 4.8 -> 4.0 ms of shading;
-// five spill and take 4.3).
+// Four resident blocks: 126-127 registers without spills, where the compiler's own
+// choice of 132-150 leaves three (shading of materials 1.47 -> 1.34 ms, Cornell 2.48
+// -> 2.16, a patterned room 8.6 -> 7.9, pattern cutouts 2.42 -> 2.22; five spill and
+// lose). Patterns with media take 128 and spill 112 bytes: 8.2-8.4 ms with either
+// number, so they keep the same rule.
 #define RT_SHADE_MIN_BLOCKS 4
 // PAT: the scene has patterns (ray cones tracked, patterned materials
 // resolved per hit). The plain instance keeps its material reads on the
@@ -1635,7 +1640,8 @@ __global__ void __launch_bounds__(BLOCK) k_sss(DevScene S, Paths P, PtConsts C, 
     st.init(stack_sh + threadIdx.x, BLOCK);
     const uint32_t n = P.cnt[CNT_SSS];
     unsigned long long rays = 0;
-    // Few walks are spread over all resident warps (lanes_for).
+    // Few walks are spread over all warps of the grid (lanes_for); the grid is the
+    // extension kernel's, of which three of five blocks are resident here.
     const uint32_t per = lanes_for(n), warp = blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5);
     const uint32_t stride = gridDim.x * (BLOCK / 32) * per;
     for (uint32_t j0 = warp * per; j0 < n; j0 += stride) {
@@ -1826,7 +1832,8 @@ __global__ void __launch_bounds__(BLOCK) k_shadow_walk(DevScene S, Paths P, PtCo
     st.init(stack_sh + threadIdx.x, BLOCK);
     const uint32_t n = P.cnt[CNT_SHADOW];
     unsigned long long rays = 0;
-    // Few paths are spread over all resident warps (lanes_for).
+    // Few paths are spread over all warps of the grid (lanes_for); the grid is the
+    // extension kernel's, of which three or four of five blocks are resident here.
     const uint32_t per = lanes_for(n), warp = blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5);
     for (uint32_t j = warp * per + lane_id(); lane_id() < per && j < n; j += gridDim.x * (BLOCK / 32) * per) {
         const uint32_t e = MED ? P.q_sh[j] : (P.q_sh[j] | SH_PRIMARY);

@@ -48,12 +48,15 @@ static const uint32_t LEAF_FIRST_MASK = (1u << 27) - 1u;
 static const int WIDE_NODE_WORDS = 6;
 
 // Leaves of a mesh hold up to four triangles (more when SAH prefers a leaf),
-// those of a mesh of up to RT_SMALL_MESH triangles up to RT_SMALL_MESH_LEAF: 32
-// leaves at most, so two levels of wide nodes still hold them, and the boxes of
-// single quads (walls, the faces of a box) are flat and turn most rays away
-// before an instance is entered. On scenes of such meshes (B200): Cornell 256
-// 2.95 -> 2.69 ms, two rooms guided 27.4 -> 25.2, media Cornell 26.9 -> 21.2;
-// meshes of thousands of triangles gain nothing from two and lose up to 5%.
+// those of a mesh of up to RT_SMALL_MESH triangles up to RT_SMALL_MESH_LEAF: the
+// boxes of single quads (walls, the faces of a box) are flat and turn most rays
+// away before an instance is entered, at the price of more leaves (up to 63 for 64
+// triangles). On scenes of meshes of 2 to 12 triangles (B200): Cornell 256 2.95 ->
+// 2.69 ms, two rooms guided 27.4 -> 25.2, media Cornell 26.9 -> 21.2; meshes of
+// thousands of triangles gain nothing from two and lose up to 5%. 400 instances of
+// one mesh, leaves of four and two: clouds of 8 triangles 7.37 and 7.08 ms, 16 13.7
+// and 12.4, 24 12.7 and 13.5, 64 16.6 and 16.3, 200 19.7 and 19.9; closed prisms of 8
+// 10.5 and 10.2, 64 11.4 both, 200 11.4 and 11.7.
 // Scenes with presence cutouts keep four everywhere: a cutout's random decision
 // hashes the triangle's place in leaf order.
 constexpr uint32_t RT_SMALL_MESH = 64, RT_SMALL_MESH_LEAF = 2;
