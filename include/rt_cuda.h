@@ -63,7 +63,7 @@ const char* rt_last_error(void);
 
 /* Gives back what the process keeps between calls and sessions: device memory
  * that destroyed sessions have returned to the library's pool, and the 16 MB
- * of pinned host memory through which results of 24 MB and more are read into
+ * of pinned host memory through which results of 16 MB and more are read into
  * pageable memory (made at the first such read). Sessions stay usable, and
  * later calls take the memory anew. */
 int rt_release_memory(void);

@@ -133,13 +133,14 @@ struct DeviceScope {
 // is in flight, so the faults and the copies run side by side. One 16 MB buffer,
 // made at the first large read-back and kept until rt_release_memory or the end of
 // the process; a call that finds it taken copies plainly. A 961 x 541 film (37 MB) came back in 8.1 ms, now 3.6;
-// below 24 MB starting the threads costs more than they save (5.5 MB: 0.4 ms more,
-// 21 MB into pages in use 1.06 ms against 1.12; 27 MB 1.34 against 1.27).
+// below 16 MB starting the threads costs more than they save (5.5 MB: 0.4 ms more).
+// 21 MB came back into fresh pages in 11.5 ms, now 4.7; into pages in use in 1.06 and
+// 1.10 on one host, in 1.29 and 1.19 on another.
 // Memory that CUDA knows (pinned, registered, managed) takes the plain copy, which
 // writes it directly: a 1920 x 1080 film (149 MB) into pinned memory 2.8 ms,
 // through the slots 5.5.
 struct ReadBack {
-    static constexpr size_t THREADS = 4, CHUNK = 2u << 20, MIN_BYTES = 24u << 20;
+    static constexpr size_t THREADS = 4, CHUNK = 2u << 20, MIN_BYTES = 16u << 20;
     // Bytes a thread copies: whole pages, and THREADS of them hold every byte.
     static constexpr size_t part(size_t bytes) { return ((bytes + THREADS - 1) / THREADS + 4095) & ~(size_t)4095; }
     std::mutex mu;
