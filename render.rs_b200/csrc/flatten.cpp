@@ -608,8 +608,8 @@ struct Collapser {
                 while (qh < 255 && (double)p[a] + qh * s < cbx.hi[a]) qh += 1;
                 qlo[a][k] = (uint8_t)ql;
                 qhi[a][k] = (uint8_t)qh;
-                // The traversal decodes fma(2^23 + q, s, p - 2^23 s) in f32;
-                // it must reproduce p + q s exactly and enclose the child.
+                // Every plane p + q s has to be an exact f32 and enclose the child
+                // (and 2^23 s a finite one, which bounds s by 2^104).
                 float sf = (float)s, p2 = p[a] - 8388608.0f * sf;
                 float dlo = std::fmaf(8388608.0f + (float)ql, sf, p2);
                 float dhi = std::fmaf(8388608.0f + (float)qh, sf, p2);
