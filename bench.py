@@ -163,16 +163,16 @@ GUIDED_W, GUIDED_H, GUIDED_SPP, GUIDED_DEPTH = 1280, 720, 2048, 16
 
 # DRAM bytes (read + write) per extension ray of k_extend on the forest, from
 # one ncu capture of all 10 k_extend launches of a 1280x720 pass of the same
-# scene (849.6 MB for 1,985,150 extension rays; 1 metric pass):
+# scene (706.8 MB for 1,985,150 extension rays; 1 metric pass):
 #   ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum,lts__t_bytes.sum
 #       --clock-control none -k regex:"k_extend" -s 10 -c 10
 #       python bench.py --mode scene --scene forest --res 1280x720 --steps 1 --warmup 1
 # A 3840x2160 launch is scaled from it by its rays; per-ray traffic falls as
 # the frame grows (582 B per ray over the first waves at 640x360), so the
 # scaled figure is an upper bound.
-EXTEND_DRAM_BYTES_PER_RAY = 849.6e6 / 1_985_150
+EXTEND_DRAM_BYTES_PER_RAY = 706.8e6 / 1_985_150
 EXTEND_DRAM_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the 10 k_extend launches of a "
-                      "1280x720 forest pass (428 B per extension ray), scaled by the rays per launch")
+                      "1280x720 forest pass (356 B per extension ray), scaled by the rays per launch")
 
 
 def rel_mse(img, ref):
@@ -705,7 +705,7 @@ def main():
             # reference traces a new ray after each, so it covers the work of
             # several reference rays.
             per_sample = work["ext_bytes_per_sample"] * samples / (ext_ms / 1e3) / 1e9
-            roof = {"kernel": "k_extend (closest hit, 8-wide BVH, cutouts decided in traversal)", "bound": "hbm",
+            roof = {"kernel": "k_extend (closest hit, 8-wide BVH, cutouts decided in traversal)", "bound": "instruction issue (frac: the reference's algorithmic bytes against HBM; L2 serves them)",
                     "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                     "traffic": EXTEND_DRAM_BYTES_PER_RAY * ext_rays / launches_ext,
                     "traffic_source": EXTEND_DRAM_SOURCE,
