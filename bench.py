@@ -705,7 +705,8 @@ def main():
             # reference traces a new ray after each, so it covers the work of
             # several reference rays.
             per_sample = work["ext_bytes_per_sample"] * samples / (ext_ms / 1e3) / 1e9
-            roof = {"kernel": "k_extend (closest hit, 8-wide BVH, cutouts decided in traversal)", "bound": "instruction issue (frac: the reference's algorithmic bytes against HBM; L2 serves them)",
+            roof = {"kernel": "k_extend (closest hit, 8-wide BVH, cutouts decided in traversal)", "bound": "hbm",
+                    "limited_by": "instruction issue; frac sets the reference's algorithmic bytes, which L2 serves, against HBM",
                     "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                     "traffic": EXTEND_DRAM_BYTES_PER_RAY * ext_rays / launches_ext,
                     "traffic_source": EXTEND_DRAM_SOURCE,
