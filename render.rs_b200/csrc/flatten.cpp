@@ -1300,13 +1300,14 @@ bool flatten_quadrics(const rt_scene_desc* d, HostScene& H, std::string* err) {
 }
 
 bool small_mesh_leaves(const rt_scene_desc* d) {
+    // Asked before the arrays are checked: what is missing is refused later.
+    if ((d->n_materials && !d->materials) || (d->n_bindings && !d->bindings)) return false;
     for (uint32_t m = 0; m < d->n_materials; m++)
         if (!(d->materials[m].presence >= 1.0)) return false;
     for (uint32_t b = 0; b < d->n_bindings; b++)
         if (d->bindings[b].field == RT_FIELD_PRESENCE) return false;
     return true;
 }
-
 
 bool flatten_scene(const rt_scene_desc* d, HostScene* out, std::string* err, bool build_bvh) {
     HostScene& H = *out;

@@ -78,6 +78,19 @@ def test_bad_max_depth_rejected():
     assert rc == -1 and "max_depth" in msg
 
 
+@pytest.mark.parametrize("build", ["host", "device"])
+@pytest.mark.parametrize("array", ["materials", "bindings", "instances", "meshes", "lights"])
+def test_missing_arrays_rejected_on_host(array, build):
+    s = scenes.patterned_room(4, 4)
+    s.add_point_light((0.0, 1.0, 0.0), 1.0)
+    d = s.desc()
+    assert getattr(d, "n_" + array) > 0
+    setattr(d, array, type(getattr(d, array))())   # the count stays
+    h, p = C.c_void_p(), abi.make_params(bvh_build=build)
+    rc = backend.lib().rt_session_create(C.byref(d), C.byref(p), C.byref(h))
+    assert rc == -1 and "NULL" in backend.lib().rt_last_error().decode()
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(backend, "_lib", None)
     monkeypatch.setattr(backend, "LIB_PATH", str(tmp_path / "nope.so"))
