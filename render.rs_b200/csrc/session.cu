@@ -132,10 +132,10 @@ struct DeviceScope {
 // its own part of the destination out of its own two slots while the next chunk
 // is in flight, so the faults and the copies run side by side. One 16 MB buffer,
 // made at the first large read-back and kept until rt_release_memory or the end of
-// the process; a call that finds it taken copies plainly. A 961 x 541 film (37 MB) came back in 8.1 ms, now 3.6;
-// below 16 MB starting the threads costs more than they save (5.5 MB: 0.4 ms more).
-// 21 MB came back into fresh pages in 11.5 ms, now 4.7; into pages in use in 1.06 and
-// 1.10 on one host, in 1.29 and 1.19 on another.
+// the process; a call that finds it taken copies plainly. A 961 x 541 film (37 MB)
+// came back in 8.1 ms, now 3.6; below 16 MB starting the threads costs more than
+// they save (5.5 MB: 0.4 ms more). 21 MB came back into fresh pages in 11.5 ms, now
+// 4.7; into pages in use in 1.06 and 1.10 on one host, in 1.29 and 1.19 on another.
 // Memory that CUDA knows (pinned, registered, managed) takes the plain copy, which
 // writes it directly: a 1920 x 1080 film (149 MB) into pinned memory 2.8 ms,
 // through the slots 5.5.
