@@ -50,25 +50,28 @@ def test_two_threads():
     assert not errors, errors
 
 
+def _best(f):
+    times = []
+    for _ in range(8):
+        t = time.perf_counter()
+        f()
+        times.append(time.perf_counter() - t)
+    return min(times)
+
+
 def test_pinned_destinations_are_written_directly():
-    """A result read into pinned memory takes one copy, not a second one through the slots: it is faster than the same
-    result read into pageable memory (twice as fast where the slots were used for both)."""
+    """A result read into pinned memory takes one copy, not a second one through the slots: about the time of that copy
+    (through the slots it took half as long again or twice as long)."""
     lib = backend.lib()
     with PtSession(scenes.cornell_box(1920, 1080), abi.make_params(max_depth=2, aovs=True)) as g:
         g.render_samples(0, 1)
         want = g.film_array()
-        pinned, pageable = torch.zeros((1080, 1920, 18), pin_memory=True).numpy(), np.zeros_like(want)
-        best = []
-        for a in (pinned, pageable):
-            times = []
-            for _ in range(8):
-                a[...] = -1.0
-                t = time.perf_counter()
-                backend._check(lib.rt_read_film(g.h, a.ctypes.data))
-                times.append(time.perf_counter() - t)
-            assert np.array_equal(a, want)
-            best.append(min(times))
-    assert best[0] < 0.8 * best[1], best
+        pinned = torch.full((1080, 1920, 18), -1.0, pin_memory=True)
+        read = _best(lambda: backend._check(lib.rt_read_film(g.h, pinned.data_ptr())))
+        assert np.array_equal(pinned.numpy(), want)
+        device = torch.zeros((1080, 1920, 18), device="cuda")
+        copy = _best(lambda: (pinned.copy_(device, non_blocking=True), torch.cuda.synchronize()))
+    assert read < 1.25 * copy + 4e-4, (read, copy)   # the film is decoded on the device first
 
 
 def test_release_memory_gives_back_and_leaves_sessions_usable():
